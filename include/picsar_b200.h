@@ -126,6 +126,26 @@ int pxrb_depose_jxjyjz(double* jx, double* jy, double* jz, int64_t np, const dou
                        int64_t nox, int64_t noy, int64_t noz, int64_t current_depo_algo,
                        int* err_flag, void* stream);
 
+/* Scratch bytes with which pxrb_depose_jxjyjz_ws puts the particles of a call
+ * (in any order) into groups and sums each group's current before its
+ * atomics; 0 where one particle per thread is the faster form (order 1, few
+ * particles, or few per group).  The contents are not kept between calls.
+ * Host function. */
+int64_t pxrb_group_scratch(int64_t order, int64_t np, int64_t nx, int64_t ny, int64_t nz,
+                           int64_t nxguard, int64_t nyguard, int64_t nzguard);
+
+/* The same with scratch (device, 4-byte aligned, at least pxrb_group_scratch
+ * bytes; NULL or less: one particle per thread).  Sums within a group are made before the atomics, so J differs
+ * by rounding. */
+int pxrb_depose_jxjyjz_ws(double* jx, double* jy, double* jz, int64_t np, const double* xp,
+                          const double* yp, const double* zp, const double* uxp,
+                          const double* uyp, const double* uzp, const double* gaminv,
+                          const double* w, double q, double xmin, double ymin, double zmin,
+                          double dt, double dx, double dy, double dz, int64_t nx, int64_t ny,
+                          int64_t nz, int64_t nxguard, int64_t nyguard, int64_t nzguard,
+                          int64_t nox, int64_t noy, int64_t noz, int64_t current_depo_algo,
+                          int* err_flag, void* scratch, int64_t scratch_bytes, void* stream);
+
 /* Replaces depose_rho_scalar_{1,2,3}_{1,2,3}_{1,2,3}
  * (src/particle_deposition/charge_deposition/charge_deposition_3d.F90:77,
  * :174, :324).  Accumulates node-centred rho. */

@@ -32,6 +32,7 @@ class PicsarB200Error(RuntimeError):
 _SIGS = {
     "pxrb_field_gathering_plus_particle_pusher": "i i" + " p" * 13 + " d" * 7 + " i" * 6
     + " p" * 6 + " d d i i d i d s",
+    "pxrb_group_scratch": "=i i i i i i i i i",
     "pxrb_geteb3d_energy_conserving": "i" + " p" * 9 + " d" * 6 + " i" * 9 + " p" * 6
     + " i i i i i s",
     "pxrb_boris_push_u_3d": "i" + " p" * 10 + " d d d d s",
@@ -39,6 +40,7 @@ _SIGS = {
     "pxrb_set_gamma": "i p p p p d s",
     "pxrb_pushxyz": "i" + " p" * 7 + " d s",
     "pxrb_depose_jxjyjz": "p p p i" + " p" * 8 + " d" * 8 + " i" * 10 + " p s",
+    "pxrb_depose_jxjyjz_ws": "p p p i" + " p" * 8 + " d" * 8 + " i" * 10 + " p p i s",
     "pxrb_depose_rho": "i p i p p p p" + " d" * 7 + " i" * 6 + " s",
     "pxrb_push_em3d_evec": " p" * 6 + " p p p" * 9 + " d d d d s",
     "pxrb_push_em3d_bvec": " p" * 6 + " p p p" * 6 + " d d d s",

@@ -2,11 +2,12 @@
 // routines, on PICSAR's own guarded column-major FP64 arrays.  One thread per
 // particle; deposition uses global FP64 atomics.  This is also the "plain
 // FP64 GPU" baseline every mixed-precision / tiled speed-up is stated against.
-#include "pxr_common.cuh"
+#include "pxr_fp64_dev.cuh"
 #include "picsar_b200.h"
 
 namespace {
 
+using namespace pxrd;
 constexpr int TPB = 256;
 
 inline int nblocks(i64 n, int tpb = TPB) {
@@ -274,115 +275,11 @@ __global__ void k_pushxyz(PushParams p) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// Esirkepov deposition with global FP64 atomics.  The old position is
-// reconstructed as x - dt/dx*ux*gaminv (esirkepov_3d.F90:161-163); for the
-// generic "_n" entry (reconstruct = 1) the new position is recomputed as
-// xold + dt/dx*v as that routine does (:3566-3577).
-// Currents are prefix sums of W along x (Jx), y (Jy), z (Jz) over the box.
-// ---------------------------------------------------------------------------
-struct DepParams {
-  i64 np;
-  const double *xp, *yp, *zp, *uxp, *uyp, *uzp, *gaminv, *w;
-  double *jx, *jy, *jz;
-  GridG G;
-  double q, xmin, ymin, zmin, dxi, dyi, dzi, dtsdx, dtsdy, dtsdz;
-  double invdtdx, invdtdy, invdtdz;
-  int reconstruct;
-  int* err;
-};
-
-template <int ORDER>
-__device__ __forceinline__ void esir_axis(double x, double xold, EsirAxis<ORDER, double>& A,
-                                          bool& ok) {
-  int n0 = EsirAxis<ORDER, double>::node(x);
-  int n1 = EsirAxis<ORDER, double>::node(xold);
-  ok = A.set(n0, x - n0, n1, xold - n1) && ok;
-}
-
 template <int ORDER>
 __global__ void __launch_bounds__(TPB) k_esirkepov(DepParams p) {
-  constexpr int M = ORDER + 2;
-  const double onethird = 1.0 / 3.0;
   for (i64 ip = blockIdx.x * (i64)blockDim.x + threadIdx.x; ip < p.np;
-       ip += (i64)gridDim.x * blockDim.x) {
-    double x = (p.xp[ip] - p.xmin) * p.dxi, y = (p.yp[ip] - p.ymin) * p.dyi,
-           z = (p.zp[ip] - p.zmin) * p.dzi;
-    double gi = p.gaminv[ip];
-    double vx = p.uxp[ip] * gi, vy = p.uyp[ip] * gi, vz = p.uzp[ip] * gi;
-    double xold = x - p.dtsdx * vx, yold = y - p.dtsdy * vy, zold = z - p.dtsdz * vz;
-    if (p.reconstruct) {
-      x = xold + p.dtsdx * vx; y = yold + p.dtsdy * vy; z = zold + p.dtsdz * vz;
-    }
-    double wq = p.q * p.w[ip];
-    double wqx = wq * p.invdtdx, wqy = wq * p.invdtdy, wqz = wq * p.invdtdz;
-    EsirAxis<ORDER, double> X, Y, Z;
-    bool ok = true;
-    esir_axis<ORDER>(x, xold, X, ok);
-    esir_axis<ORDER>(y, yold, Y, ok);
-    esir_axis<ORDER>(z, zold, Z, ok);
-    if (!ok) { atomicExch(p.err, 1); continue; }
-    // Jx: sweep x for every (j, k)
-#pragma unroll
-    for (int k = 0; k < M; ++k) {
-      if (k >= Z.n) continue;
-      double dsz = Z.s1[k] - Z.s0[k];
-#pragma unroll
-      for (int j = 0; j < M; ++j) {
-        if (j >= Y.n) continue;
-        double dsy = Y.s1[j] - Y.s0[j];
-        double fyz = (Y.s0[j] + 0.5 * dsy) * Z.s0[k] + (0.5 * Y.s0[j] + onethird * dsy) * dsz;
-        double acc = 0.0;
-        double* row = p.jx + p.G.idx(X.i0, Y.i0 + j, Z.i0 + k);
-#pragma unroll
-        for (int i = 0; i < M - 1; ++i) {
-          if (i >= X.n - 1) continue;
-          acc = acc + wqx * (X.s1[i] - X.s0[i]) * fyz;
-          atomicAdd(row + i, acc);
-        }
-      }
-    }
-    // Jy: sweep y for every (i, k)
-#pragma unroll
-    for (int k = 0; k < M; ++k) {
-      if (k >= Z.n) continue;
-      double dsz = Z.s1[k] - Z.s0[k];
-#pragma unroll
-      for (int i = 0; i < M; ++i) {
-        if (i >= X.n) continue;
-        double dsx = X.s1[i] - X.s0[i];
-        double fzx = (Z.s0[k] + 0.5 * dsz) * X.s0[i] + (0.5 * Z.s0[k] + onethird * dsz) * dsx;
-        double acc = 0.0;
-        double* col = p.jy + p.G.idx(X.i0 + i, Y.i0, Z.i0 + k);
-#pragma unroll
-        for (int j = 0; j < M - 1; ++j) {
-          if (j >= Y.n - 1) continue;
-          acc = acc + wqy * (Y.s1[j] - Y.s0[j]) * fzx;
-          atomicAdd(col + j * p.G.sx, acc);
-        }
-      }
-    }
-    // Jz: sweep z for every (i, j)
-#pragma unroll
-    for (int j = 0; j < M; ++j) {
-      if (j >= Y.n) continue;
-      double dsy = Y.s1[j] - Y.s0[j];
-#pragma unroll
-      for (int i = 0; i < M; ++i) {
-        if (i >= X.n) continue;
-        double dsx = X.s1[i] - X.s0[i];
-        double fxy = (X.s0[i] + 0.5 * dsx) * Y.s0[j] + (0.5 * X.s0[i] + onethird * dsx) * dsy;
-        double acc = 0.0;
-        double* col = p.jz + p.G.idx(X.i0 + i, Y.i0 + j, Z.i0);
-#pragma unroll
-        for (int k = 0; k < M - 1; ++k) {
-          if (k >= Z.n - 1) continue;
-          acc = acc + wqz * (Z.s1[k] - Z.s0[k]) * fxy;
-          atomicAdd(col + k * p.G.sy, acc);
-        }
-      }
-    }
-  }
+       ip += (i64)gridDim.x * blockDim.x)
+    deposit_one<ORDER>(p, ip);
 }
 
 // Node-centred charge deposition (charge_deposition_3d.F90:77-400).
@@ -913,14 +810,14 @@ int pxrb_pushxyz(int64_t np, double* xp, double* yp, double* zp, const double* u
                      nullptr, nullptr, nullptr, nullptr, xp, yp, zp, 0, 1, dt, 1, 0, stream);
 }
 
-int pxrb_depose_jxjyjz(double* jx, double* jy, double* jz, int64_t np, const double* xp,
+int pxrb_depose_jxjyjz_ws(double* jx, double* jy, double* jz, int64_t np, const double* xp,
                        const double* yp, const double* zp, const double* uxp,
                        const double* uyp, const double* uzp, const double* gaminv,
                        const double* w, double q, double xmin, double ymin, double zmin,
                        double dt, double dx, double dy, double dz, int64_t nx, int64_t ny,
                        int64_t nz, int64_t nxguard, int64_t nyguard, int64_t nzguard,
                        int64_t nox, int64_t noy, int64_t noz, int64_t current_depo_algo,
-                       int* err_flag, void* stream) {
+                       int* err_flag, void* scratch, int64_t scratch_bytes, void* stream) {
   if (np < 0) return PXRB_EINVAL;
   if (np == 0) return PXRB_OK;
   if (nox != noy || noy != noz || nox < 1 || nox > 3) return PXRB_EUNSUPPORTED;
@@ -939,12 +836,28 @@ int pxrb_depose_jxjyjz(double* jx, double* jy, double* jz, int64_t np, const dou
   p.reconstruct = current_depo_algo == 1;
   p.err = err_flag;
   cudaStream_t s = (cudaStream_t)stream;
+  if (group_fits((int)nox, np, p.G, scratch, scratch_bytes))
+    return esirkepov_grouped((int)nox, p, scratch, s);
   int nb = nblocks(np);
   if (nox == 1) k_esirkepov<1><<<nb, TPB, 0, s>>>(p);
   else if (nox == 2) k_esirkepov<2><<<nb, TPB, 0, s>>>(p);
   else k_esirkepov<3><<<nb, TPB, 0, s>>>(p);
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
+}
+
+int pxrb_depose_jxjyjz(double* jx, double* jy, double* jz, int64_t np, const double* xp,
+                       const double* yp, const double* zp, const double* uxp,
+                       const double* uyp, const double* uzp, const double* gaminv,
+                       const double* w, double q, double xmin, double ymin, double zmin,
+                       double dt, double dx, double dy, double dz, int64_t nx, int64_t ny,
+                       int64_t nz, int64_t nxguard, int64_t nyguard, int64_t nzguard,
+                       int64_t nox, int64_t noy, int64_t noz, int64_t current_depo_algo,
+                       int* err_flag, void* stream) {
+  return pxrb_depose_jxjyjz_ws(jx, jy, jz, np, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin,
+                               ymin, zmin, dt, dx, dy, dz, nx, ny, nz, nxguard, nyguard,
+                               nzguard, nox, noy, noz, current_depo_algo, err_flag, nullptr, 0,
+                               stream);
 }
 
 int pxrb_depose_rho(int64_t order, double* rho, int64_t np, const double* xp,

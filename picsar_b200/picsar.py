@@ -916,6 +916,19 @@ def pxr_pushxyz(np_, xp, yp, zp, uxp, uyp, uzp, gaminv, dt):
               float(dt), _stream())
 
 
+def _group_scratch(order, np_, nx, ny, nz, gx, gy, gz, device):
+    """(tensor, pointer, bytes) of the scratch the grouped deposition takes
+    for a call, (None, None, 0) where one particle per thread is used."""
+    if np_ < 1 << 16:             # pxrb_group_scratch is 0 (spares small calls the query)
+        return None, None, 0
+    need = _lib.query("pxrb_group_scratch", int(order), int(np_), int(nx), int(ny), int(nz),
+                      int(gx), int(gy), int(gz))
+    if need <= 0:
+        return None, None, 0
+    t = torch.empty(need, dtype=torch.uint8, device=device)
+    return t, t.data_ptr(), need
+
+
 def depose_jxjyjz(jx, jy, jz, np_, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin, ymin, zmin,
                   dt, dx, dy, dz, nx, ny, nz, nxguard, nyguard, nzguard, nox, noy, noz,
                   current_depo_algo=0, err_flag=None):
@@ -924,12 +937,14 @@ def depose_jxjyjz(jx, jy, jz, np_, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin
     own = err_flag is None
     if own:
         err_flag = torch.zeros(1, dtype=torch.int32, device=jx.device)
-    _lib.call("pxrb_depose_jxjyjz", *[_ptr(a, grid=True) for a in (jx, jy, jz)], int(np_),
+    keep, scr, nscr = (_group_scratch(nox, np_, nx, ny, nz, nxguard, nyguard, nzguard, jx.device)
+                       if nox == noy == noz else (None, None, 0))
+    _lib.call("pxrb_depose_jxjyjz_ws", *[_ptr(a, grid=True) for a in (jx, jy, jz)], int(np_),
               *[_ptr(a) for a in (xp, yp, zp, uxp, uyp, uzp, gaminv, w)], float(q),
               float(xmin), float(ymin), float(zmin), float(dt), float(dx), float(dy), float(dz),
               int(nx), int(ny), int(nz), int(nxguard), int(nyguard), int(nzguard), int(nox),
               int(noy), int(noz), int(current_depo_algo),
-              _ptr(err_flag, "err_flag", dtype=torch.int32), _stream())
+              _ptr(err_flag, "err_flag", dtype=torch.int32), scr, nscr, _stream())
 
 
 def depose_jxjyjz_esirkepov(jx, jy, jz, np_, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin,

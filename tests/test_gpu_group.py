@@ -1,0 +1,72 @@
+"""The grouped deposition (particles put into groups, FP64 matrix products) against one particle per thread, on the same inputs: odd
+sizes, each order and pusher, particles in no order and in the guard cells,
+exact half-way positions, node changes along every axis, batches that are
+not full."""
+import numpy as np
+import pytest
+import torch
+
+from picsar_b200 import _lib
+from picsar_b200 import picsar as P
+
+pytestmark = pytest.mark.gpu
+
+G = 4
+
+
+def _inputs(n, np_, seed, spread):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    r = lambda *s: torch.rand(*s, generator=g, device="cuda", dtype=torch.float64)
+    x = [(r(np_) * (v + 2) - 1) for v in n]                # one cell into the guards
+    for a in x:
+        a[: np_ // 8] = torch.round(a[: np_ // 8] * 2) / 2  # nodes and half-way points
+    u = [spread * (r(np_) - 0.5) for _ in range(3)]
+    w = r(np_) + 0.5
+    fields = []
+    for _ in range(6):
+        f = P.grid_zeros(*n, G)
+        f.copy_(r(*f.shape) - 0.5)
+        fields.append(f)
+    return x, u, w, fields
+
+
+def _scratch(order, np_, n):
+    # what pxrb_group_scratch would return without its size rule: an upper
+    # bound of keys, chunks and three ints per particle
+    keys = (n[0] + 2 * G + 8) * (n[1] + 2 * G + 1) * (n[2] + 2 * G + 1)
+    return torch.empty(4 * (2 * keys + 64 + 3 * np_) + 256, dtype=torch.uint8, device="cuda")
+
+
+@pytest.mark.parametrize("order", [1, 2, 3])
+@pytest.mark.parametrize("algo,np_,spread", [(0, 20011, 0.4), (1, 997, 1.5), (0, 1, 0.1)])
+def test_deposit_matches_one_particle_per_thread(cuda, order, algo, np_, spread):
+    n, dt = (19, 13, 11), 0.5
+    x, u, w, _ = _inputs(n, np_, 20 * order + algo, spread)
+    gi = 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = []
+    for scr in (None, _scratch(order, np_, n)):
+        j = [P.grid_zeros(*n, G) for _ in range(3)]
+        for a in j:
+            a.fill_(0.125)                                  # the deposition accumulates
+        _lib.call("pxrb_depose_jxjyjz_ws", *[a.data_ptr() for a in j], np_,
+                  *[a.data_ptr() for a in x + u], gi.data_ptr(), w.data_ptr(), -1.0, 0.0, 0.0,
+                  0.0, dt, 1.0, 1.0, 1.0, *n, G, G, G, order, order, order, algo, err.data_ptr(),
+                  None if scr is None else scr.data_ptr(), 0 if scr is None else scr.numel(),
+                  torch.cuda.current_stream().cuda_stream)
+        out.append(j)
+    assert int(err.item()) == 0
+    per_node = max(1.0, np_ / (n[0] * n[1] * n[2]) * 64)
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) <= 64 * per_node * 2.3e-16
+
+
+def test_scratch_rule(cuda):
+    """No scratch where the grouped form is not used; enough where it is."""
+    q = lambda np_, n: _lib.query("pxrb_group_scratch", 3, np_, n, n, n, 3, 3, 3)
+    assert q(1000, 16) == 0
+    assert q(1 << 16, 512) == 0
+    big = q(1 << 20, 64)
+    assert big >= 4 * (3 * (1 << 20) + 71 * 71 * 15)
+    assert np.iinfo(np.int32).max > big
