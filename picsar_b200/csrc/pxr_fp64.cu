@@ -105,67 +105,37 @@ __global__ void __launch_bounds__(TPB) k_gather_push(GPParams p) {
 }
 
 // Separate gather (geteb3d_energy_conserving), both l_lower_order_in_v
-// branches and the nodal switch; accumulates.  Generic over the order with
-// run-time shapes (the scalar Fortran forms, field_gathering_o{1,2,3}_3d.F90).
-struct Sh {
-  int i0, n;
-  double s[4];
+// branches and the nodal switch; accumulates.  One kernel per order and
+// branch: with run-time orders the shapes sat in local memory and the point
+// loops did not unroll.
+//
+// Staggered shape of degree DEG at x - ss (ss = 1/2, or 0 on the nodal grid):
+// the scalar Fortran forms, field_gathering_o{1,2,3}_3d.F90.
+template <int DEG> struct StagDeg {
+  static constexpr int N = DEG + 1;
+  int i0;
+  double s[N];
+  __device__ __forceinline__ void set(double x, double ss) {
+    if (DEG == 0) {
+      i0 = ffloor(x + 0.5 - ss); s[0] = 1.0;
+    } else if (DEG == 1) {
+      const int j0 = ffloor(x - ss);
+      const double xi = x - ss - j0;
+      i0 = j0; s[0] = 1.0 - xi; s[1] = xi;
+    } else if (DEG == 2) {
+      const int j0 = ffloor(x + 0.5 - ss);
+      const double xi = x - ss - j0, xs = xi * xi;
+      i0 = j0 - 1;
+      s[0] = 0.5 * (0.5 - xi) * (0.5 - xi); s[1] = 0.75 - xs; s[2] = 0.5 * (0.5 + xi) * (0.5 + xi);
+    } else {
+      const int j0 = ffloor(x - ss);
+      const double xi = x - ss - j0, ox = 1.0 - xi, xs = xi * xi, oxs = ox * ox;
+      i0 = j0 - 1;
+      s[0] = (1.0 / 6.0) * oxs * ox; s[1] = (2.0 / 3.0) - xs * (1.0 - xi * 0.5);
+      s[2] = (2.0 / 3.0) - oxs * (1.0 - ox * 0.5); s[3] = (1.0 / 6.0) * xs * xi;
+    }
+  }
 };
-
-__device__ __forceinline__ void sh_node(int order, double x, Sh& r) {
-  if (order == 1) {
-    int j = (int)floor(x); double xi = x - j;
-    r.i0 = j; r.n = 2; r.s[0] = 1.0 - xi; r.s[1] = xi;
-  } else if (order == 2) {
-    int j = (int)round(x); double xi = x - j, xs = xi * xi;
-    r.i0 = j - 1; r.n = 3;
-    r.s[0] = 0.5 * (0.5 - xi) * (0.5 - xi); r.s[1] = 0.75 - xs; r.s[2] = 0.5 * (0.5 + xi) * (0.5 + xi);
-  } else {
-    int j = (int)floor(x); double xi = x - j, ox = 1.0 - xi, xs = xi * xi, oxs = ox * ox;
-    r.i0 = j - 1; r.n = 4;
-    r.s[0] = (1.0 / 6.0) * oxs * ox; r.s[1] = (2.0 / 3.0) - xs * (1.0 - xi * 0.5);
-    r.s[2] = (2.0 / 3.0) - oxs * (1.0 - ox * 0.5); r.s[3] = (1.0 / 6.0) * xs * xi;
-  }
-}
-
-__device__ __forceinline__ void sh_stag(int order, bool lower, double ss, double x, Sh& r) {
-  if (order == 1) {
-    if (lower) { r.i0 = (int)floor(x + 0.5 - ss); r.n = 1; r.s[0] = 1.0; }
-    else {
-      int j0 = (int)floor(x - ss); double xi = x - ss - j0;
-      r.i0 = j0; r.n = 2; r.s[0] = 1.0 - xi; r.s[1] = xi;
-    }
-  } else if (order == 2) {
-    if (lower) {
-      int j0 = (int)floor(x - ss); double xi = x - ss - j0;
-      r.i0 = j0; r.n = 2; r.s[0] = 1.0 - xi; r.s[1] = xi;
-    } else {
-      int j0 = (int)floor(x + 0.5 - ss); double xi = x - ss - j0, xs = xi * xi;
-      r.i0 = j0 - 1; r.n = 3;
-      r.s[0] = 0.5 * (0.5 - xi) * (0.5 - xi); r.s[1] = 0.75 - xs; r.s[2] = 0.5 * (0.5 + xi) * (0.5 + xi);
-    }
-  } else {
-    if (lower) {
-      int j0 = (int)floor(x + 0.5 - ss); double xi = x - ss - j0, xs = xi * xi;
-      r.i0 = j0 - 1; r.n = 3;
-      r.s[0] = 0.5 * (0.5 - xi) * (0.5 - xi); r.s[1] = 0.75 - xs; r.s[2] = 0.5 * (0.5 + xi) * (0.5 + xi);
-    } else {
-      int j0 = (int)floor(x - ss); double xi = x - ss - j0, ox = 1.0 - xi, xs = xi * xi, oxs = ox * ox;
-      r.i0 = j0 - 1; r.n = 4;
-      r.s[0] = (1.0 / 6.0) * oxs * ox; r.s[1] = (2.0 / 3.0) - xs * (1.0 - xi * 0.5);
-      r.s[2] = (2.0 / 3.0) - oxs * (1.0 - ox * 0.5); r.s[3] = (1.0 / 6.0) * xs * xi;
-    }
-  }
-}
-
-__device__ __forceinline__ double gsum(const double* g, const GridG& G, const Sh& a,
-                                       const Sh& b, const Sh& c, double f) {
-  for (int ll = 0; ll < c.n; ++ll)
-    for (int kk = 0; kk < b.n; ++kk)
-      for (int jj = 0; jj < a.n; ++jj)
-        f = f + a.s[jj] * b.s[kk] * c.s[ll] * __ldg(g + G.idx(a.i0 + jj, b.i0 + kk, c.i0 + ll));
-  return f;
-}
 
 struct GEBParams {
   i64 np;
@@ -174,27 +144,26 @@ struct GEBParams {
   double xmin, ymin, zmin, dxi, dyi, dzi;
   const double *exg, *eyg, *ezg, *bxg, *byg, *bzg;
   GridG G;
-  int order, lower;
   double ss;
 };
 
+template <int ORDER, bool LOWER>
 __global__ void __launch_bounds__(TPB) k_geteb(GEBParams p) {
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < p.np;
-       i += (i64)gridDim.x * blockDim.x) {
-    double x = (p.xp[i] - p.xmin) * p.dxi, y = (p.yp[i] - p.ymin) * p.dyi,
-           z = (p.zp[i] - p.zmin) * p.dzi;
-    Sh nx, ny, nz, sx, sy, sz;
-    sh_node(p.order, x, nx); sh_node(p.order, y, ny); sh_node(p.order, z, nz);
-    sh_stag(p.order, p.lower, p.ss, x, sx);
-    sh_stag(p.order, p.lower, p.ss, y, sy);
-    sh_stag(p.order, p.lower, p.ss, z, sz);
-    p.ex[i] = gsum(p.exg, p.G, sx, ny, nz, p.ex[i]);
-    p.ey[i] = gsum(p.eyg, p.G, nx, sy, nz, p.ey[i]);
-    p.ez[i] = gsum(p.ezg, p.G, nx, ny, sz, p.ez[i]);
-    p.bx[i] = gsum(p.bxg, p.G, nx, sy, sz, p.bx[i]);
-    p.by[i] = gsum(p.byg, p.G, sx, ny, sz, p.by[i]);
-    p.bz[i] = gsum(p.bzg, p.G, sx, sy, nz, p.bz[i]);
-  }
+  constexpr int N = ORDER + 1, DEG = LOWER ? ORDER - 1 : ORDER, S = DEG + 1;
+  const i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+  if (i >= p.np) return;
+  const double x = (p.xp[i] - p.xmin) * p.dxi, y = (p.yp[i] - p.ymin) * p.dyi,
+               z = (p.zp[i] - p.zmin) * p.dzi;
+  NodeShape<ORDER, double> nx, ny, nz;
+  StagDeg<DEG> sx, sy, sz;
+  nx.set(x); ny.set(y); nz.set(z);
+  sx.set(x, p.ss); sy.set(y, p.ss); sz.set(z, p.ss);
+  p.ex[i] = gather_comp<S, N, N>(p.exg, p.G, sx.i0, sx.s, ny.i0, ny.s, nz.i0, nz.s, p.ex[i]);
+  p.ey[i] = gather_comp<N, S, N>(p.eyg, p.G, nx.i0, nx.s, sy.i0, sy.s, nz.i0, nz.s, p.ey[i]);
+  p.ez[i] = gather_comp<N, N, S>(p.ezg, p.G, nx.i0, nx.s, ny.i0, ny.s, sz.i0, sz.s, p.ez[i]);
+  p.bx[i] = gather_comp<N, S, S>(p.bxg, p.G, nx.i0, nx.s, sy.i0, sy.s, sz.i0, sz.s, p.bx[i]);
+  p.by[i] = gather_comp<S, N, S>(p.byg, p.G, sx.i0, sx.s, ny.i0, ny.s, sz.i0, sz.s, p.by[i]);
+  p.bz[i] = gather_comp<S, S, N>(p.bzg, p.G, sx.i0, sx.s, sy.i0, sy.s, nz.i0, nz.s, p.bz[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -461,11 +430,17 @@ struct G2 {
   __device__ __forceinline__ i64 idx(i64 i, i64 k) const { return (i + gx) + sx * (k + gz); }
 };
 
-__device__ __forceinline__ double gsum2(const double* g, const G2& G, const Sh& a, const Sh& c,
-                                        double f) {
-  for (int ll = 0; ll < c.n; ++ll)
-    for (int jj = 0; jj < a.n; ++jj)
-      f = f + a.s[jj] * c.s[ll] * __ldg(g + G.idx(a.i0 + jj, c.i0 + ll));
+template <int NA, int NC>
+__device__ __forceinline__ double gather2(const double* __restrict__ g, const G2& G, int ia,
+                                          const double* sa, int ic, const double* sc, double f) {
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const double* row = g + G.idx(ia, ic + c);
+    double r = 0.0;
+#pragma unroll
+    for (int t = 0; t < NA; ++t) r = r + sa[t] * __ldg(row + t);
+    f = f + r * sc[c];
+  }
   return f;
 }
 
@@ -476,24 +451,25 @@ struct GEB2Params {
   double xmin, zmin, dxi, dzi;
   const double *exg, *eyg, *ezg, *bxg, *byg, *bzg;
   G2 G;
-  int order, lower;
   double ss;
 };
 
+template <int ORDER, bool LOWER>
 __global__ void __launch_bounds__(TPB) k_geteb2d(GEB2Params p) {
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < p.np;
-       i += (i64)gridDim.x * blockDim.x) {
-    const double x = (p.xp[i] - p.xmin) * p.dxi, z = (p.zp[i] - p.zmin) * p.dzi;
-    Sh nx, nz, sx, sz;
-    sh_node(p.order, x, nx); sh_node(p.order, z, nz);
-    sh_stag(p.order, p.lower, p.ss, x, sx); sh_stag(p.order, p.lower, p.ss, z, sz);
-    p.ex[i] = gsum2(p.exg, p.G, sx, nz, p.ex[i]);
-    p.ey[i] = gsum2(p.eyg, p.G, nx, nz, p.ey[i]);
-    p.ez[i] = gsum2(p.ezg, p.G, nx, sz, p.ez[i]);
-    p.bx[i] = gsum2(p.bxg, p.G, nx, sz, p.bx[i]);
-    p.by[i] = gsum2(p.byg, p.G, sx, sz, p.by[i]);
-    p.bz[i] = gsum2(p.bzg, p.G, sx, nz, p.bz[i]);
-  }
+  constexpr int N = ORDER + 1, DEG = LOWER ? ORDER - 1 : ORDER, S = DEG + 1;
+  const i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+  if (i >= p.np) return;
+  const double x = (p.xp[i] - p.xmin) * p.dxi, z = (p.zp[i] - p.zmin) * p.dzi;
+  NodeShape<ORDER, double> nx, nz;
+  StagDeg<DEG> sx, sz;
+  nx.set(x); nz.set(z);
+  sx.set(x, p.ss); sz.set(z, p.ss);
+  p.ex[i] = gather2<S, N>(p.exg, p.G, sx.i0, sx.s, nz.i0, nz.s, p.ex[i]);
+  p.ey[i] = gather2<N, N>(p.eyg, p.G, nx.i0, nx.s, nz.i0, nz.s, p.ey[i]);
+  p.ez[i] = gather2<N, S>(p.ezg, p.G, nx.i0, nx.s, sz.i0, sz.s, p.ez[i]);
+  p.bx[i] = gather2<N, S>(p.bxg, p.G, nx.i0, nx.s, sz.i0, sz.s, p.bx[i]);
+  p.by[i] = gather2<S, S>(p.byg, p.G, sx.i0, sx.s, sz.i0, sz.s, p.by[i]);
+  p.bz[i] = gather2<S, N>(p.bzg, p.G, sx.i0, sx.s, nz.i0, nz.s, p.bz[i]);
 }
 
 struct Dep2Params {
@@ -505,83 +481,97 @@ struct Dep2Params {
 };
 
 // The reference's 2-D shapes: order 3 with its default-real (single
-// precision) constants 1/6 and 2/3; array index off = shift of the shape.
-template <int ORDER>
-__device__ __forceinline__ void shape2d(double xint, double* s, int off) {
+// precision) constants 1/6 and 2/3.
+template <int ORDER> __device__ __forceinline__ void shape2d(double xint, double* s) {
   if (ORDER == 1) {
-    s[0 + off] = 1.0 - xint; s[1 + off] = xint;
+    s[0] = 1.0 - xint; s[1] = xint;
   } else if (ORDER == 2) {
     const double xs = xint * xint;
-    s[-1 + off] = 0.5 * (0.5 - xint) * (0.5 - xint);
-    s[0 + off] = 0.75 - xs;
-    s[1 + off] = 0.5 * (0.5 + xint) * (0.5 + xint);
+    s[0] = 0.5 * (0.5 - xint) * (0.5 - xint);
+    s[1] = 0.75 - xs;
+    s[2] = 0.5 * (0.5 + xint) * (0.5 + xint);
   } else {
     const double onesixth = (double)(1.0f / 6.0f), twothird = (double)(2.0f / 3.0f);
     const double ox = 1.0 - xint, xs = xint * xint, oxs = ox * ox;
-    s[-1 + off] = onesixth * oxs * ox;
-    s[0 + off] = twothird - xs * (1.0 - xint * 0.5);
-    s[1 + off] = twothird - oxs * (1.0 - ox * 0.5);
-    s[2 + off] = onesixth * xs * xint;
+    s[0] = onesixth * oxs * ox;
+    s[1] = twothird - xs * (1.0 - xint * 0.5);
+    s[2] = twothird - oxs * (1.0 - ox * 0.5);
+    s[3] = onesixth * xs * xint;
   }
 }
 
+// One axis: the new (s0) and old (s1) shapes on the common box of their
+// nodes, every index a compile-time constant (with shape arrays indexed by
+// the run-time shift the kernel worked out of local memory).
+template <int ORDER> struct Box2 {
+  static constexpr int M = ORDER + 2;
+  i64 i0;                   // first node of the box
+  int n;
+  double s0[M], d[M];       // new shape; old minus new
+  __device__ __forceinline__ void set(double x, double xold) {
+    const i64 n0 = ORDER == 2 ? (i64)round(x) : (i64)floor(x);
+    const i64 n1 = ORDER == 2 ? (i64)round(xold) : (i64)floor(xold);
+    double t0[ORDER + 1], t1[ORDER + 1];
+    shape2d<ORDER>(x - n0, t0);
+    shape2d<ORDER>(xold - n1, t1);
+    // a move of more than one cell per step (beyond the CFL limit) would
+    // leave the box: clamp, as no valid input reaches it
+    int s = (int)(n1 - n0);
+    s = s < -1 ? -1 : (s > 1 ? 1 : s);
+    const bool up0 = s < 0, up1 = s > 0;
+    i0 = n0 - ORDER / 2 - (up0 ? 1 : 0);
+    n = ORDER + 1 + (s != 0 ? 1 : 0);
+#pragma unroll
+    for (int r = 0; r < M; ++r) {
+      const double a0 = r <= ORDER ? t0[r <= ORDER ? r : 0] : 0.0, b0 = r ? t0[r ? r - 1 : 0] : 0.0;
+      const double a1 = r <= ORDER ? t1[r <= ORDER ? r : 0] : 0.0, b1 = r ? t1[r ? r - 1 : 0] : 0.0;
+      s0[r] = up0 ? b0 : a0;
+      d[r] = (up1 ? b1 : a1) - s0[r];
+    }
+  }
+};
+
+// A warp takes particles SPREAD apart: neighbours in memory are mostly in one
+// cell, and atomics of many lanes to one address go one by one.
 template <int ORDER>
 __global__ void __launch_bounds__(TPB) k_esirkepov2d(Dep2Params p) {
-  constexpr int a = ORDER == 1 ? 0 : 1, b = ORDER == 3 ? 2 : 1;
+  constexpr int M = ORDER + 2, SPREAD = TPB / 32;
   const double onethird = (double)(1.0f / 3.0f);
   const double dxi = 1.0 / p.dx, dzi = 1.0 / p.dz;
   const double dtsdx0 = p.dt * dxi, dtsdz0 = p.dt * dzi;
   const double invvol = 1.0 / (p.dx * p.dz), invdtdx = 1.0 / (p.dt * p.dz),
                invdtdz = 1.0 / (p.dt * p.dx);
-  for (i64 ip = blockIdx.x * (i64)blockDim.x + threadIdx.x; ip < p.np;
-       ip += (i64)gridDim.x * blockDim.x) {
-    // (-2:3) arrays at offset +2
-    double sx_[6] = {0, 0, 0, 0, 0, 0}, sz_[6] = {0, 0, 0, 0, 0, 0};
-    double sx0_[6] = {0, 0, 0, 0, 0, 0}, sz0_[6] = {0, 0, 0, 0, 0, 0};
-    double sdzk_[6] = {0, 0, 0, 0, 0, 0}, sdzkm1_[6] = {0, 0, 0, 0, 0, 0};
-    double *sx = sx_ + 2, *sz = sz_ + 2, *sx0 = sx0_ + 2, *sz0 = sz0_ + 2;
-    double *sdzk = sdzk_ + 2, *sdzkm1 = sdzkm1_ + 2;
-    const double x = (p.xp[ip] - p.xmin) * dxi, z = (p.zp[ip] - p.zmin) * dzi;
-    const double gi = p.gaminv[ip];
-    const double vx = p.uxp[ip] * gi, vy = p.uyp[ip] * gi, vz = p.uzp[ip] * gi;
-    const double xold = x - dtsdx0 * vx, zold = z - dtsdz0 * vz;
-    const double wq = p.q * p.w[ip], wqx = wq * invdtdx, wqz = wq * invdtdz;
-    const i64 iixp0 = ORDER == 2 ? (i64)round(x) : (i64)floor(x);
-    const i64 ikxp0 = ORDER == 2 ? (i64)round(z) : (i64)floor(z);
-    shape2d<ORDER>(x - iixp0, sx0, 0);
-    shape2d<ORDER>(z - ikxp0, sz0, 0);
-    const i64 iixp = ORDER == 2 ? (i64)round(xold) : (i64)floor(xold);
-    const i64 ikxp = ORDER == 2 ? (i64)round(zold) : (i64)floor(zold);
-    int dix = (int)(iixp - iixp0), diz = (int)(ikxp - ikxp0);
-    // a move of more than one cell per step (beyond the CFL limit) would
-    // leave the shape arrays: clamp, as no valid input reaches it
-    dix = dix < -1 ? -1 : (dix > 1 ? 1 : dix);
-    diz = diz < -1 ? -1 : (diz > 1 ? 1 : diz);
-    shape2d<ORDER>(xold - iixp, sx, dix);
-    shape2d<ORDER>(zold - ikxp, sz, diz);
-    const int ixmin = min(0, dix) - a, ixmax = max(0, dix) + b;
-    const int izmin = min(0, diz) - a, izmax = max(0, diz) + b;
-    double sdxi = 0.0, sdxim1 = 0.0;
-    for (int k = izmin; k <= izmax; ++k) {
-      const double dsz = sz[k] - sz0[k];
-      for (int i = ixmin; i <= ixmax; ++i) {
-        const double dsx = sx[i] - sx0[i];
-        const i64 c = p.G.idx(iixp0 + i, ikxp0 + k);
-        if (i < ixmax) {
-          sdxi = wqx * dsx * (sz0[k] + 0.5 * dsz);
-          if (i > ixmin) sdxi = sdxi + sdxim1;
-          atomicAdd(p.jx + c, sdxi);
-        }
-        atomicAdd(p.jy + c, wq * vy * invvol *
-                                ((sz0[k] + 0.5 * dsz) * sx0[i] + (0.5 * sz0[k] + onethird * dsz) * dsx));
-        if (k < izmax) {
-          sdzk[i] = wqz * dsz * (sx0[i] + 0.5 * dsx);
-          if (k > izmin) sdzk[i] = sdzk[i] + sdzkm1[i];
-          atomicAdd(p.jz + c, sdzk[i]);
-        }
-        sdxim1 = sdxi;
+  const i64 ip = blockIdx.x * (i64)TPB + (threadIdx.x & 31) * SPREAD + (threadIdx.x >> 5);
+  if (ip >= p.np) return;
+  const double x = (p.xp[ip] - p.xmin) * dxi, z = (p.zp[ip] - p.zmin) * dzi;
+  const double gi = p.gaminv[ip];
+  const double vx = p.uxp[ip] * gi, vy = p.uyp[ip] * gi, vz = p.uzp[ip] * gi;
+  const double wq = p.q * p.w[ip], wqx = wq * invdtdx, wqz = wq * invdtdz;
+  Box2<ORDER> X, Z;
+  X.set(x, x - dtsdx0 * vx);
+  Z.set(z, z - dtsdz0 * vz);
+  const i64 c0 = p.G.idx(X.i0, Z.i0);
+  double cz[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) cz[i] = 0.0;
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    if (k >= Z.n) continue;
+    double cx = 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      if (i >= X.n) continue;
+      const i64 c = c0 + i + p.G.sx * k;
+      if (i < X.n - 1) {
+        cx = cx + wqx * X.d[i] * (Z.s0[k] + 0.5 * Z.d[k]);
+        atomicAdd(p.jx + c, cx);
       }
-      for (int t = 0; t < 6; ++t) sdzkm1_[t] = sdzk_[t];
+      atomicAdd(p.jy + c, wq * vy * invvol * ((Z.s0[k] + 0.5 * Z.d[k]) * X.s0[i] +
+                                              (0.5 * Z.s0[k] + onethird * Z.d[k]) * X.d[i]));
+      if (k < Z.n - 1) {
+        cz[i] = cz[i] + wqz * Z.d[k] * (X.s0[i] + 0.5 * X.d[i]);
+        atomicAdd(p.jz + c, cz[i]);
+      }
     }
   }
 }
@@ -742,9 +732,14 @@ int pxrb_geteb3d_energy_conserving(
   p.dxi = 1.0 / dx; p.dyi = 1.0 / dy; p.dzi = 1.0 / dz;
   p.exg = exg; p.eyg = eyg; p.ezg = ezg; p.bxg = bxg; p.byg = byg; p.bzg = bzg;
   p.G = make_grid(nx, ny, nz, nxguard, nyguard, nzguard);
-  p.order = (int)nox; p.lower = l_lower_order_in_v != 0;
   p.ss = l_nodal ? 0.0 : 0.5;
-  k_geteb<<<nblocks(np), TPB, 0, (cudaStream_t)stream>>>(p);
+  cudaStream_t s = (cudaStream_t)stream;
+  const int nb = nblocks(np);
+#define PXRB_GEB(O_)                                                  \
+  if (l_lower_order_in_v) k_geteb<O_, true><<<nb, TPB, 0, s>>>(p);    \
+  else k_geteb<O_, false><<<nb, TPB, 0, s>>>(p);
+  if (nox == 1) { PXRB_GEB(1) } else if (nox == 2) { PXRB_GEB(2) } else { PXRB_GEB(3) }
+#undef PXRB_GEB
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
 }
@@ -1029,9 +1024,14 @@ int pxrb_geteb2dxz_energy_conserving(
   p.xmin = xmin; p.zmin = zmin; p.dxi = 1.0 / dx; p.dzi = 1.0 / dz;
   p.exg = exg; p.eyg = eyg; p.ezg = ezg; p.bxg = bxg; p.byg = byg; p.bzg = bzg;
   p.G.gx = nxguard; p.G.gz = nzguard; p.G.sx = nx + 1 + 2 * nxguard;
-  p.order = (int)nox; p.lower = l_lower_order_in_v ? 1 : 0;
   p.ss = l_nodal ? 0.0 : 0.5;
-  k_geteb2d<<<nblocks(np), TPB, 0, (cudaStream_t)stream>>>(p);
+  cudaStream_t s = (cudaStream_t)stream;
+  const int nb = nblocks(np);
+#define PXRB_GEB(O_)                                                    \
+  if (l_lower_order_in_v) k_geteb2d<O_, true><<<nb, TPB, 0, s>>>(p);    \
+  else k_geteb2d<O_, false><<<nb, TPB, 0, s>>>(p);
+  if (nox == 1) { PXRB_GEB(1) } else if (nox == 2) { PXRB_GEB(2) } else { PXRB_GEB(3) }
+#undef PXRB_GEB
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
 }
