@@ -25,12 +25,13 @@ __device__ __forceinline__ double gather_comp(const double* __restrict__ g, cons
                                               int ia, const double* sa, int ib,
                                               const double* sb, int ic, const double* sc,
                                               double f) {
+  const double* base = g + G.idx(ia, ib, ic);
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     double a = 0.0;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      const double* row = g + G.idx(ia, ib + b, ic + c);
+      const double* row = base + (G.sx * b + G.sy * c);
       double r = 0.0;
 #pragma unroll
       for (int t = 0; t < NA; ++t) r = r + sa[t] * __ldg(row + t);
@@ -74,8 +75,19 @@ struct GPParams {
 // field_gathering_plus_particle_pusher_{n}_{n}_{n}: gather (+=) into the
 // particle field arrays, then Boris + set_gamma (pusher 0) or Vay (1), then
 // pushxyz, all with the module time step dt.
+// Blocks of 128 threads, as many per SM as the gather's registers allow: left
+// to itself the compiler took 136 registers at order 3, one block of 256 per
+// SM.  8.4 M particles in cell order, fused gather + push: order 3 2255 ->
+// 1019 us, order 2 971 -> 712 us (order 1 keeps the 64 registers it had,
+// 350 us); 5 or 6 blocks at order 3 spill (1067, 1114 us).
+constexpr int GTPB = 128;
+constexpr int gp_blocks(int order) { return order == 1 ? 8 : 4; }
+// separate gather, same particles, lower / full shapes: order 3 1497 / 2304 ->
+// 744 / 1288 us, order 2 814 / 901 -> 528 / 617 us
+constexpr int geteb_blocks(int order, bool lower) { return order == 3 ? (lower ? 5 : 4) : 6; }
+
 template <int ORDER, int PUSHER>
-__global__ void __launch_bounds__(TPB) k_gather_push(GPParams p) {
+__global__ void __launch_bounds__(GTPB, gp_blocks(ORDER)) k_gather_push(GPParams p) {
   const double cst_b = p.q * p.dt * 0.5 / p.m;
   const double cst_v = p.q * p.dt / p.m;
   const double clghtisq = 1.0 / (p.clight * p.clight);
@@ -148,7 +160,7 @@ struct GEBParams {
 };
 
 template <int ORDER, bool LOWER>
-__global__ void __launch_bounds__(TPB) k_geteb(GEBParams p) {
+__global__ void __launch_bounds__(GTPB, geteb_blocks(ORDER, LOWER)) k_geteb(GEBParams p) {
   constexpr int N = ORDER + 1, DEG = LOWER ? ORDER - 1 : ORDER, S = DEG + 1;
   const i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   if (i >= p.np) return;
@@ -678,11 +690,11 @@ int pxrb_field_gathering_plus_particle_pusher(
   p.G = make_grid(nx, ny, nz, nxguard, nyguard, nzguard);
   p.q = q; p.m = m; p.dt = dt; p.clight = clight;
   cudaStream_t s = (cudaStream_t)stream;
-  int nb = nblocks(np);
+  int nb = nblocks(np, GTPB);
   int vay = particle_pusher == 1;
 #define LAUNCH_GP(O)                                                                   \
-  if (vay) k_gather_push<O, 1><<<nb, TPB, 0, s>>>(p);                                  \
-  else k_gather_push<O, 0><<<nb, TPB, 0, s>>>(p);
+  if (vay) k_gather_push<O, 1><<<nb, GTPB, 0, s>>>(p);                                  \
+  else k_gather_push<O, 0><<<nb, GTPB, 0, s>>>(p);
   if (order == 1) { LAUNCH_GP(1) }
   else if (order == 2) { LAUNCH_GP(2) }
   else { LAUNCH_GP(3) }
@@ -734,10 +746,10 @@ int pxrb_geteb3d_energy_conserving(
   p.G = make_grid(nx, ny, nz, nxguard, nyguard, nzguard);
   p.ss = l_nodal ? 0.0 : 0.5;
   cudaStream_t s = (cudaStream_t)stream;
-  const int nb = nblocks(np);
+  const int nb = nblocks(np, GTPB);
 #define PXRB_GEB(O_)                                                  \
-  if (l_lower_order_in_v) k_geteb<O_, true><<<nb, TPB, 0, s>>>(p);    \
-  else k_geteb<O_, false><<<nb, TPB, 0, s>>>(p);
+  if (l_lower_order_in_v) k_geteb<O_, true><<<nb, GTPB, 0, s>>>(p);    \
+  else k_geteb<O_, false><<<nb, GTPB, 0, s>>>(p);
   if (nox == 1) { PXRB_GEB(1) } else if (nox == 2) { PXRB_GEB(2) } else { PXRB_GEB(3) }
 #undef PXRB_GEB
   PXRB_CHECK_LAUNCH();
