@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K,
   typedef Geom<ORDER> GE;
   typedef EsirAxis<ORDER, double> AX;
   extern __shared__ __align__(16) unsigned char smem[];
-  double* buf = reinterpret_cast<double*>(smem + (threadIdx.x >> 5) * GE::WARP_BYTES_DEPOSIT);
+  double* buf = reinterpret_cast<double*>(smem + (threadIdx.x >> 5) * GE::WARP_BYTES);
   Group g;
   if (!group_of<ORDER>(K, s, p.np, g)) return;               // whole warp
   const int lane = threadIdx.x & 31;
@@ -206,8 +206,11 @@ __global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K,
 #pragma unroll
       for (int t = 0; t < GE::N + 1; ++t) X.s0[t] = X.s1[t] = 0.0;
     }
-    J.add(buf, X, sy0, sy1, sz0, sz1, X.i0 - (g.bx - GE::A), f * p.invdtdx, f * p.invdtdy,
-          f * p.invdtdz, (n + 3) >> 2);
+    J.stage(buf, X, sy0, sy1, sz0, sz1, f * p.invdtdx, f * p.invdtdy, f * p.invdtdz);
+    __syncwarp();
+#pragma unroll 1
+    for (int t = 0; t < (n + 3) >> 2; ++t) J.sub(buf, t, X.i0 - (g.bx - GE::A));
+    __syncwarp();
   }
   const GridG& G = p.G;
   const int nx0 = g.bx - GE::A, ny0 = g.by - GE::A, nz0 = g.bz - GE::A;
@@ -278,7 +281,7 @@ template <class KERN> int big_smem(KERN k, int bytes) {
 template <int ORDER>
 int run_esirkepov(const DepParams& p, const Keys& K, const Scratch& s, cudaStream_t st) {
   PosParams q = {p.np, p.xp, p.yp, p.zp, p.xmin, p.ymin, p.zmin, p.dxi, p.dyi, p.dzi};
-  const int smem = WARPS * Geom<ORDER>::WARP_BYTES_DEPOSIT;
+  const int smem = WARPS * Geom<ORDER>::WARP_BYTES;
   if (const int e = big_smem(k_esirkepov_group<ORDER>, smem)) return e;
   if (const int e = group_particles<ORDER>(q, K, s, st)) return e;
   k_esirkepov_group<ORDER><<<(K.nkeys + WARPS - 1) / WARPS, TPB, smem, st>>>(p, K, s);

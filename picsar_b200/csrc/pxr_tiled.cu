@@ -28,7 +28,7 @@ int launch_order2(int, int, int, int, const pxrb_tiled_job*, const int2*, int, c
 int launch_order3(int, int, int, int, const pxrb_tiled_job*, const int2*, int, const int*, int*, int, int, size_t, cudaStream_t);
 }  // namespace pxrt
 
-#include "pxr_tiled_kernel.cuh"
+#include "pxr_tile_group.cuh"
 
 namespace {
 using namespace pxrt;
@@ -782,6 +782,12 @@ int64_t smem_bytes(int order, int prec, int acc, int tx, int ty, int tz, int dri
   const i64 V = (i64)pxrt::win_sz(tx, W) * W;
   i64 r = prec ? 8 : 4;
   i64 a = acc == 3 ? 8 : 4, nw = acc == 2 ? 2 : 1;
+  if (prec == 1 && order == 3) {      // grouped FP64 kernel
+    if (tx == 8 && drift == 1) return pxrt::TileGroups<3, 8, 1>::SMEM;
+    if (tx == 8 && drift == 0) return pxrt::TileGroups<3, 8, 0>::SMEM;
+    if (tx == 4 && drift == 1) return pxrt::TileGroups<3, 4, 1>::SMEM;
+    if (tx == 4 && drift == 0) return pxrt::TileGroups<3, 4, 0>::SMEM;
+  }
   const i64 hb = tx + 2 * drift;      // next-step occupancy histogram (fixed point)
   if (acc == 4)                       // cell-grouped kernel (cg_smem_bytes)
     return V * 36 + hb * hb * hb * 12 + 4 + ((hb * hb * hb * 2 + 15) / 16) * 16 + 256 * 8;

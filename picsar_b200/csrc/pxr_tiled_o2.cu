@@ -23,7 +23,7 @@ int launch_shape(int tile, int drift, int mode, const Job* jobs, const int2* wor
   if (tile == T_ && drift == D_ && mode == M_)                                              \
     return launch_step<R, ORDER, T_, D_, M_>(jobs, work, nwork, nwork_dev, ctr, threads,    \
                                              ctas, smem, s);
-  if (sizeof(R) == 8) {
+  if constexpr (sizeof(R) == 8) {
     PXRB_TD(8, 1, 3)
     PXRB_TD(8, 0, 3)
     PXRB_TD(4, 1, 3)

@@ -1,5 +1,6 @@
 // Instantiations of the fused particle kernel for shape order 3.
 #include "pxr_cell_kernel.cuh"
+#include "pxr_tile_group.cuh"
 
 namespace pxrt {
 template <typename R, int ORDER, int T, int D, int MODE>
@@ -19,21 +20,24 @@ template <typename R, int ORDER>
 int launch_shape(int tile, int drift, int mode, const Job* jobs, const int2* work, int nwork,
                  const int* nwork_dev, int* ctr, int threads, int ctas, size_t smem,
                  cudaStream_t s) {
+#define PXRB_TG(T_, D_)                                                                      \
+  if (tile == T_ && drift == D_ && mode == 3)                                               \
+    return launch_group<ORDER, T_, D_>(jobs, work, nwork, nwork_dev, ctr, threads, ctas, smem, s);
 #define PXRB_TD(T_, D_, M_)                                                                  \
   if (tile == T_ && drift == D_ && mode == M_)                                              \
     return launch_step<R, ORDER, T_, D_, M_>(jobs, work, nwork, nwork_dev, ctr, threads,    \
                                              ctas, smem, s);
   if (mode == 4) {       // cell-grouped kernel (FP32, int32 fixed point)
-    if (sizeof(R) != 4) return PXRB_EUNSUPPORTED;
+    if constexpr (sizeof(R) != 4) return PXRB_EUNSUPPORTED;
     if (tile == 8 && drift == 1)
       return launch_cell<ORDER, 8, 1>(jobs, work, nwork, nwork_dev, ctr, threads, ctas, smem, s);
     return PXRB_EUNSUPPORTED;
   }
-  if (sizeof(R) == 8) {
-    PXRB_TD(8, 1, 3)
-    PXRB_TD(8, 0, 3)
-    PXRB_TD(4, 1, 3)
-    PXRB_TD(4, 0, 3)
+  if constexpr (sizeof(R) == 8) {
+    PXRB_TG(8, 1)
+    PXRB_TG(8, 0)
+    PXRB_TG(4, 1)
+    PXRB_TG(4, 0)
   } else {
     PXRB_TD(8, 1, 2)
     PXRB_TD(8, 1, 1)
@@ -46,6 +50,7 @@ int launch_shape(int tile, int drift, int mode, const Job* jobs, const int2* wor
     PXRB_TD(4, 0, 2)
   }
 #undef PXRB_TD
+#undef PXRB_TG
   return PXRB_EUNSUPPORTED;
 }
 

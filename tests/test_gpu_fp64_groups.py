@@ -1,0 +1,33 @@
+"""The FP64 engine's grouped order-3 particle kernel against the oracle where
+its groups can go wrong."""
+import numpy as np
+import pytest
+
+from picsar_b200.tiled import TiledConfig
+from tests._cases import random_fields, rel_l2
+from tests.test_gpu_tiled import _pair
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,tile,drift,crowd", [((20, 11, 17), 8, 1, 0), ((16, 16, 16), 8, 1, 3000),
+                                                ((13, 18, 9), 4, 0, 0), ((24, 16, 8), 8, 0, 0)])
+def test_tiled_fp64_groups_at_the_edges(cuda, n, tile, drift, crowd):
+    """The FP64 order-3 kernel's groups: partial tiles, cells with none or
+    thousands of particles, fast particles that leave their group, their
+    tile window or the box, over steps without a sort."""
+    rng = np.random.default_rng(sum(n))
+    m = 3 * n[0] * n[1] * n[2]
+    st = {c: rng.uniform(0, L, m) for c, L in zip("xyz", n)}
+    for c in "xyz":
+        st[c][:crowd] = 3.0 + rng.uniform(0, 1, crowd)
+        st["u" + c] = 0.6 * rng.standard_normal(m)
+    st["w"] = 0.01 * rng.uniform(0.5, 1.5, m)
+    cfg = TiledConfig(tile=(tile,) * 3, drift=drift, sort_interval=0, relayout_interval=0)
+    o, t = _pair(n, 3, 1, "fp64", st, cfg, random_fields(n, 3, 5))
+    for _ in range(3):
+        o.step(1)
+        t.step(1, keep_j=True)
+    assert t.error_flag() == 0
+    for name in ("jx", "jy", "jz", "ex", "by"):
+        assert rel_l2(t.export_field(name, 3).cpu().numpy(), o.get_field(name)) <= 1e-12, name
