@@ -342,33 +342,39 @@ constexpr int RR_MAXC = 512;        // cells per tile (tile edge <= 8)
 // moves the particles into the *_b buffers in destination order, and those
 // trade places with the particle arrays in the descriptors.
 
-// One warp per tile: classes numbered in input order with per-class counters
-// in shared memory (no block barriers), then the destination of every
-// particle from the level table, stored as the source of that destination.
+// One CTA per tile: classes numbered in input order, then the destination of
+// every particle from the level table, stored as the source of that
+// destination.  The tile is taken in segments, each split into one run per
+// warp: the runs' class counts are summed first, so that each warp numbers
+// its run on its own.  (With one warp per tile the numbering was a serial
+// chain over the tile.  8 warps against one: re-layout of 32^3 cells at 8 per
+// cell 87 -> 23 us, 128x128x64 256 -> 202, 192^3 1274 -> 1247; sort 134 -> 50,
+// 388 -> 314, 2111 -> 1910 us, with FP64 at order 2 809 -> 438.)
 // CELL_MAJOR: the input order is the sort's cell-major permutation (perm);
 // otherwise the tile's current order.  Scratch: rank_b (level and class per
 // input slot); output: cell_b (source particle per destination).
-constexpr int TM_WARPS = 4;         // tiles per CTA
-constexpr int TM_LEVELS = 256;      // level table entries per tile
-constexpr int TM_SEG = 4096;        // classes staged per tile segment
+constexpr int TM_WARPS = 8, TM_TPB = 32 * TM_WARPS;
+constexpr int TM_LEVELS = 256;      // level table entries
+constexpr int TM_SEG = 4096;        // classes staged per segment
 
 template <typename R, bool CELL_MAJOR>
-__global__ void __launch_bounds__(TM_WARPS * 32) k_tile_map(const Job* __restrict__ jp) {
-  __shared__ int s_cnt[TM_WARPS][32];
-  __shared__ int s_P[TM_WARPS][TM_LEVELS];
-  __shared__ unsigned s_M[TM_WARPS][TM_LEVELS];
-  __shared__ unsigned char s_cls[TM_WARPS][TM_SEG];
+__global__ void __launch_bounds__(TM_TPB) k_tile_map(const Job* __restrict__ jp) {
+  __shared__ int cnt[32];                      // particles numbered so far, per class
+  __shared__ int s_run[TM_WARPS][32];          // per run: counts, then first levels
+  __shared__ int s_P[TM_LEVELS];
+  __shared__ unsigned s_M[TM_LEVELS];
+  __shared__ unsigned char cls[TM_SEG];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const Job& J = jp[blockIdx.y];
-  const int t = blockIdx.x * TM_WARPS + wid;
+  const int t = blockIdx.x;
   const int ntl = J.ntx * J.nty * J.ntz;
-  if (t >= ntl) return;                       // whole warp
+  if (t >= ntl) return;
   const int b0 = J.tile_off[t], b1 = J.tile_off[t + 1];
   if (b0 == b1) return;
   if (J.cell_order) {
     // cell order: the sort's permutation as it is; a re-layout keeps the
     // current order (the cell-grouped kernel groups by cell itself)
-    for (int i = b0 + lane; i < b1; i += 32)
+    for (int i = b0 + threadIdx.x; i < b1; i += TM_TPB)
       J.cell_b[i] = CELL_MAJOR ? (uint32_t)J.perm[i] : (uint32_t)i;
     return;
   }
@@ -387,7 +393,6 @@ __global__ void __launch_bounds__(TM_WARPS * 32) k_tile_map(const Job* __restric
   const int* __restrict__ perm = J.perm;
   int* key_at = J.rank_b;
   uint32_t* src_at = J.cell_b;
-  int* cnt = s_cnt[wid];
   auto source = [&](int sl) { return CELL_MAJOR ? __ldg(perm + sl) : sl; };
   // class of a particle from its current cell (window-relative, periodic)
   auto class_of = [&](int p) {
@@ -404,30 +409,33 @@ __global__ void __launch_bounds__(TM_WARPS * 32) k_tile_map(const Job* __restric
     return (x + SY * y + SZ * z) & 31;
   };
   const bool packed = b1 - b0 < (1 << 26);    // level and class in one int
-  cnt[lane] = 0;
-  // per segment: the classes first (independent loads, several in flight)
-  // into shared memory, then the numbering pass over them in order
-  constexpr int U = 4;
-  unsigned char* cls = s_cls[wid];
+  if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
   for (int seg = b0; seg < b1; seg += TM_SEG) {
     const int sn = min(TM_SEG, b1 - seg);
-    for (int i0 = 0; i0 < sn; i0 += 32 * U) {
-      int kk[U];
+    s_run[wid][lane] = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < sn; i += TM_TPB) cls[i] = (unsigned char)class_of(source(seg + i));
+    __syncthreads();
+    // this warp's run: a multiple of 32 slots
+    const int len = ((sn + TM_TPB - 1) / TM_TPB) * 32;
+    const int r0 = min(wid * len, sn), r1 = min(r0 + len, sn);
+    for (int i = r0 + lane; i < r1; i += 32) atomicAdd(&s_run[wid][cls[i]], 1);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      int run = cnt[threadIdx.x];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + 32 * u + lane;
-        kk[u] = i < sn ? class_of(source(seg + i)) : 0;
+      for (int w = 0; w < TM_WARPS; ++w) {
+        const int c = s_run[w][threadIdx.x];
+        s_run[w][threadIdx.x] = run;
+        run += c;
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + 32 * u + lane;
-        if (i < sn) cls[i] = (unsigned char)kk[u];
-      }
+      cnt[threadIdx.x] = run;
     }
-    __syncwarp();
-    for (int base = 0; base < sn; base += 32) {
+    __syncthreads();
+    int* at = s_run[wid];
+    for (int base = r0; base < r1; base += 32) {
       const int i = base + lane;
-      const bool valid = i < sn;
+      const bool valid = i < r1;
       const int k = valid ? (int)cls[i] : 0;
       // lanes of the same class: five ballots over the class bits
       unsigned peers = __ballot_sync(0xffffffffu, valid);
@@ -436,13 +444,13 @@ __global__ void __launch_bounds__(TM_WARPS * 32) k_tile_map(const Job* __restric
         const unsigned m = __ballot_sync(0xffffffffu, (k >> b) & 1);
         peers &= ((k >> b) & 1) ? m : ~m;
       }
-      const int lev = valid ? cnt[k] + __popc(peers & ((1u << lane) - 1u)) : 0;
+      const int lev = valid ? at[k] + __popc(peers & ((1u << lane) - 1u)) : 0;
       __syncwarp();
-      if (valid && lane == __ffs(peers) - 1) cnt[k] += __popc(peers);
+      if (valid && lane == __ffs(peers) - 1) at[k] += __popc(peers);
       __syncwarp();
       if (valid) key_at[seg + i] = packed ? (lev << 5 | k) : lev;
     }
-    __syncwarp();
+    __syncthreads();
   }
   int nmax = cnt[lane];
 #pragma unroll
@@ -458,25 +466,26 @@ __global__ void __launch_bounds__(TM_WARPS * 32) k_tile_map(const Job* __restric
     }
   };
   if (table) {
-    for (int l = lane; l < nmax; l += 32) level_row(l, s_P[wid][l], s_M[wid][l]);
-    __syncwarp();
+    for (int l = threadIdx.x; l < nmax; l += TM_TPB) level_row(l, s_P[l], s_M[l]);
+    __syncthreads();
   }
-  for (int s0 = b0; s0 < b1; s0 += 32 * U) {
+  constexpr int U = 4;
+  for (int s0 = b0; s0 < b1; s0 += TM_TPB * U) {
     int kv[U], pp[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int sl = s0 + 32 * u + lane;
+      const int sl = s0 + TM_TPB * u + threadIdx.x;
       kv[u] = sl < b1 ? key_at[sl] : 0;
       pp[u] = sl < b1 ? source(sl) : 0;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int sl = s0 + 32 * u + lane;
+      const int sl = s0 + TM_TPB * u + threadIdx.x;
       if (sl >= b1) continue;
       const int lev = packed ? kv[u] >> 5 : kv[u], k = packed ? kv[u] & 31 : class_of(pp[u]);
       int P;
       unsigned M;
-      if (table) { P = s_P[wid][lev]; M = s_M[wid][lev]; }
+      if (table) { P = s_P[lev]; M = s_M[lev]; }
       else level_row(lev, P, M);
       src_at[b0 + P + __popc(M & ((1u << k) - 1u))] = (uint32_t)pp[u];
     }
@@ -890,10 +899,10 @@ int pxrb_tiled_sort(const pxrb_tiled_job* job_host, pxrb_tiled_job* job_dev, voi
     if (!J.perm) return PXRB_EINVAL;
     k_sort_perm<<<nb, 256, 0, s>>>(job_dev);
     if (J.prec == 0) {
-      k_tile_map<float, true><<<(ntiles + TM_WARPS - 1) / TM_WARPS, TM_WARPS * 32, 0, s>>>(job_dev);
+      k_tile_map<float, true><<<ntiles, TM_TPB, 0, s>>>(job_dev);
       k_relayout_gather<float><<<nb, 256, 0, s>>>(job_dev);
     } else {
-      k_tile_map<double, true><<<(ntiles + TM_WARPS - 1) / TM_WARPS, TM_WARPS * 32, 0, s>>>(job_dev);
+      k_tile_map<double, true><<<ntiles, TM_TPB, 0, s>>>(job_dev);
       k_relayout_gather<double><<<nb, 256, 0, s>>>(job_dev);
     }
     k_swap_particle_buffers<<<1, 32, 0, s>>>(job_dev, 1);
@@ -921,10 +930,10 @@ int pxrb_tiled_sort_batch(pxrb_tiled_job* jobs_dev, int32_t njobs, int32_t prec,
   k_sort_scan<<<g_one, SCAN_TPB, 0, s>>>(jobs_dev);
   k_sort_perm<<<g_np, 256, 0, s>>>(jobs_dev);
   if (prec == 0) {
-    k_tile_map<float, true><<<dim3((max_tiles + TM_WARPS - 1) / TM_WARPS, njobs), TM_WARPS * 32, 0, s>>>(jobs_dev);
+    k_tile_map<float, true><<<dim3(max_tiles, njobs), TM_TPB, 0, s>>>(jobs_dev);
     k_relayout_gather<float><<<g_np, 256, 0, s>>>(jobs_dev);
   } else {
-    k_tile_map<double, true><<<dim3((max_tiles + TM_WARPS - 1) / TM_WARPS, njobs), TM_WARPS * 32, 0, s>>>(jobs_dev);
+    k_tile_map<double, true><<<dim3(max_tiles, njobs), TM_TPB, 0, s>>>(jobs_dev);
     k_relayout_gather<double><<<g_np, 256, 0, s>>>(jobs_dev);
   }
   k_swap_particle_buffers<<<(njobs + 127) / 128, 128, 0, s>>>(jobs_dev, njobs);
@@ -942,12 +951,12 @@ int pxrb_tiled_relayout(pxrb_tiled_job* jobs_dev, int32_t njobs, int32_t prec,
   const int64_t want = (max_np + 255) / 256;
   const int cap = njobs >= 4096 ? 1 : 4096 / njobs;
   const int bx = (int)std::max<int64_t>(1, std::min<int64_t>(want, cap));
-  const dim3 g_tiles((max_tiles + TM_WARPS - 1) / TM_WARPS, njobs), g_np(bx, njobs);
+  const dim3 g_tiles(max_tiles, njobs), g_np(bx, njobs);
   if (prec == 0) {
-    k_tile_map<float, false><<<g_tiles, TM_WARPS * 32, 0, s>>>(jobs_dev);
+    k_tile_map<float, false><<<g_tiles, TM_TPB, 0, s>>>(jobs_dev);
     k_relayout_gather<float><<<g_np, 256, 0, s>>>(jobs_dev);
   } else {
-    k_tile_map<double, false><<<g_tiles, TM_WARPS * 32, 0, s>>>(jobs_dev);
+    k_tile_map<double, false><<<g_tiles, TM_TPB, 0, s>>>(jobs_dev);
     k_relayout_gather<double><<<g_np, 256, 0, s>>>(jobs_dev);
   }
   k_swap_particle_buffers<<<(njobs + 127) / 128, 128, 0, s>>>(jobs_dev, njobs);
