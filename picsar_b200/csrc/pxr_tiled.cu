@@ -49,19 +49,35 @@ __device__ __forceinline__ int find_job(const int64_t* off, int njobs, int64_t g
   return lo;
 }
 
-template <typename R>
-__device__ __forceinline__ void store_images(R* base, int i, int j, int k, int nx, int ny,
-                                             int nz, int G, int pitch, int NYg, R v) {
-  int ii[2] = {i, 0}, jj[2] = {j, 0}, kk[2] = {k, 0};
-  int ni = 1, nj = 1, nk = 1;
-  if (i < G) ii[ni++] = i + nx; else if (i >= nx - G) ii[ni++] = i - nx;
-  if (j < G) jj[nj++] = j + ny; else if (j >= ny - G) jj[nj++] = j - ny;
-  if (k < G) kk[nk++] = k + nz; else if (k >= nz - G) kk[nk++] = k - nz;
-  for (int c = 0; c < nk; ++c)
-    for (int b = 0; b < nj; ++b)
-      for (int a = 0; a < ni; ++a)
-        base[(ii[a] + G) + (i64)pitch * ((jj[b] + G) + (i64)NYg * (kk[c] + G))] = v;
-}
+// v to element c (cell i, j, k) and its periodic images in the guards; each
+// axis has at least 2 G cells, so a cell has at most one image per axis.
+// (Predicated stores at precomputed offsets: with index arrays and loop
+// counts the addresses went through local memory.)
+struct Images {
+  i64 x, y, z;                        // offsets of the images, 0: none
+  __device__ __forceinline__ Images(int i, int j, int k, int nx, int ny, int nz, int G, i64 sy,
+                                    i64 sz) {
+    x = i < G ? nx : (i >= nx - G ? -nx : 0);
+    y = (j < G ? ny : (j >= ny - G ? -ny : 0)) * sy;
+    z = (k < G ? nz : (k >= nz - G ? -nz : 0)) * sz;
+  }
+  template <typename R> __device__ __forceinline__ void store(R* p, R v) const {
+    p[0] = v;
+    if (x) p[x] = v;
+    if (y) {
+      p[y] = v;
+      if (x) p[x + y] = v;
+    }
+    if (z) {
+      p[z] = v;
+      if (x) p[x + z] = v;
+      if (y) {
+        p[y + z] = v;
+        if (x) p[x + y + z] = v;
+      }
+    }
+  }
+};
 
 // Cell (i, j, k) of a job's flat cell index (x fastest).  The flat index of
 // one job is below 2^32 (2^32 cells of the engine's layout exceed any one
@@ -75,18 +91,21 @@ __device__ __forceinline__ void yee_ijk(int64_t lid, int nx, int ny, int& i, int
   k = (int)kk;
 }
 
-// Each thread updates YEE_CPT cells spaced by the block size, loading all of
-// them before computing (memory-level parallelism); a block covers YEE_CPB
-// consecutive cells of one job.
+// Each thread updates CPT cells spaced by the block size, loading all of them
+// before computing (memory-level parallelism); a block covers YEE_TPB * CPT
+// consecutive cells of one job.  Jobs start at multiples of YEE_CPB cells.
 constexpr int YEE_CPT = 4;
 constexpr int YEE_CPB = YEE_TPB * YEE_CPT;
+// One cell per thread where four would leave SMs without a block (B push 32^3
+// 5.7 -> 2.8 us, 64^3 6.9 -> 5.3; 96^3, with four, 12.9 -> 12.2 by the stores).
+constexpr i64 YEE_SMALL = (i64)YEE_CPB * 148 * 2;
 
-template <typename R>
+template <typename R, int CPT>
 __global__ void __launch_bounds__(YEE_TPB)
     k_yee_b_t(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ off, R frac) {
   __shared__ int s_job;
   __shared__ R s_c[3];
-  const int64_t gid0 = (int64_t)blockIdx.x * YEE_CPB;
+  const int64_t gid0 = (int64_t)blockIdx.x * (YEE_TPB * CPT);
   if (threadIdx.x == 0) {
     const int jb = find_job(off, njobs, gid0);
     const Job& J0 = jobs[jb];
@@ -105,10 +124,10 @@ __global__ void __launch_bounds__(YEE_TPB)
   const R* ex = (const R*)J.ex; const R* ey = (const R*)J.ey; const R* ez = (const R*)J.ez;
   R* bx = (R*)J.bx; R* by = (R*)J.by; R* bz = (R*)J.bz;
   const R dtsdx = s_c[0], dtsdy = s_c[1], dtsdz = s_c[2];
-  int ci[YEE_CPT], cj[YEE_CPT], ck[YEE_CPT];
-  R vbx[YEE_CPT], vby[YEE_CPT], vbz[YEE_CPT];
+  int ci[CPT], cj[CPT], ck[CPT];
+  R vbx[CPT], vby[CPT], vbz[CPT];
 #pragma unroll
-  for (int u = 0; u < YEE_CPT; ++u) {
+  for (int u = 0; u < CPT; ++u) {
     const int64_t lid = l0 + u * YEE_TPB;
     if (lid < ncell) {
       yee_ijk(lid, nx, ny, ci[u], cj[u], ck[u]);
@@ -120,22 +139,24 @@ __global__ void __launch_bounds__(YEE_TPB)
     }
   }
 #pragma unroll
-  for (int u = 0; u < YEE_CPT; ++u) {
+  for (int u = 0; u < CPT; ++u) {
     if (l0 + u * YEE_TPB < ncell) {
-      store_images(bx, ci[u], cj[u], ck[u], nx, ny, nz, G, pitch, NYg, vbx[u]);
-      store_images(by, ci[u], cj[u], ck[u], nx, ny, nz, G, pitch, NYg, vby[u]);
-      store_images(bz, ci[u], cj[u], ck[u], nx, ny, nz, G, pitch, NYg, vbz[u]);
+      const i64 c = (ci[u] + G) + sy * (cj[u] + G) + sz * (ck[u] + G);
+      const Images im(ci[u], cj[u], ck[u], nx, ny, nz, G, sy, sz);
+      im.store(bx + c, vbx[u]);
+      im.store(by + c, vby[u]);
+      im.store(bz + c, vbz[u]);
     }
   }
 }
 
-template <typename R>
+template <typename R, int CPT>
 __global__ void __launch_bounds__(YEE_TPB)
     k_yee_e_t(const Job* __restrict__ jobs, int njobs, const int64_t* __restrict__ off,
               int zero_j) {
   __shared__ int s_job;
   __shared__ R s_c[4];
-  const int64_t gid0 = (int64_t)blockIdx.x * YEE_CPB;
+  const int64_t gid0 = (int64_t)blockIdx.x * (YEE_TPB * CPT);
   if (threadIdx.x == 0) {
     const int jb = find_job(off, njobs, gid0);
     const Job& J0 = jobs[jb];
@@ -157,10 +178,10 @@ __global__ void __launch_bounds__(YEE_TPB)
   const R* bx = (const R*)J.bx; const R* by = (const R*)J.by; const R* bz = (const R*)J.bz;
   double* jxp = J.jx; double* jyp = J.jy; double* jzp = J.jz;
   const R mudt = s_c[0], dtsdx = s_c[1], dtsdy = s_c[2], dtsdz = s_c[3];
-  int ci[YEE_CPT], cj[YEE_CPT], ck[YEE_CPT];
-  R vex[YEE_CPT], vey[YEE_CPT], vez[YEE_CPT];
+  int ci[CPT], cj[CPT], ck[CPT];
+  R vex[CPT], vey[CPT], vez[CPT];
 #pragma unroll
-  for (int u = 0; u < YEE_CPT; ++u) {
+  for (int u = 0; u < CPT; ++u) {
     const int64_t lid = l0 + u * YEE_TPB;
     if (lid < ncell) {
       yee_ijk(lid, nx, ny, ci[u], cj[u], ck[u]);
@@ -173,13 +194,15 @@ __global__ void __launch_bounds__(YEE_TPB)
     }
   }
 #pragma unroll
-  for (int u = 0; u < YEE_CPT; ++u) {
+  for (int u = 0; u < CPT; ++u) {
     const int64_t lid = l0 + u * YEE_TPB;
     if (lid < ncell) {
       if (zero_j) { jxp[lid] = 0.0; jyp[lid] = 0.0; jzp[lid] = 0.0; }
-      store_images(ex, ci[u], cj[u], ck[u], nx, ny, nz, G, pitch, NYg, vex[u]);
-      store_images(ey, ci[u], cj[u], ck[u], nx, ny, nz, G, pitch, NYg, vey[u]);
-      store_images(ez, ci[u], cj[u], ck[u], nx, ny, nz, G, pitch, NYg, vez[u]);
+      const i64 c = (ci[u] + G) + sy * (cj[u] + G) + sz * (ck[u] + G);
+      const Images im(ci[u], cj[u], ck[u], nx, ny, nz, G, sy, sz);
+      im.store(ex + c, vex[u]);
+      im.store(ey + c, vey[u]);
+      im.store(ez + c, vez[u]);
     }
   }
 }
@@ -850,10 +873,14 @@ int pxrb_tiled_push_b(const pxrb_tiled_job* jobs_dev, int32_t njobs, int32_t pre
   if (!jobs_dev || !cell_off_dev || njobs < 1 || total_cells < 0 || total_cells % YEE_CPB)
     return PXRB_EINVAL;
   if (total_cells == 0) return PXRB_OK;
-  int nb = (int)(total_cells / YEE_CPB);
+  const bool small = total_cells < YEE_SMALL;
+  const int nb = (int)(total_cells / (small ? YEE_TPB : YEE_CPB));
   cudaStream_t s = (cudaStream_t)stream;
-  if (prec == 0) k_yee_b_t<float><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, (float)frac);
-  else k_yee_b_t<double><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, frac);
+#define PXRB_YEE(R_)                                                                               \
+  if (small) k_yee_b_t<R_, 1><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, (R_)frac);    \
+  else k_yee_b_t<R_, YEE_CPT><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, (R_)frac);
+  if (prec == 0) { PXRB_YEE(float) } else { PXRB_YEE(double) }
+#undef PXRB_YEE
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
 }
@@ -864,10 +891,14 @@ int pxrb_tiled_push_e(const pxrb_tiled_job* jobs_dev, int32_t njobs, int32_t pre
   if (!jobs_dev || !cell_off_dev || njobs < 1 || total_cells < 0 || total_cells % YEE_CPB)
     return PXRB_EINVAL;
   if (total_cells == 0) return PXRB_OK;
-  int nb = (int)(total_cells / YEE_CPB);
+  const bool small = total_cells < YEE_SMALL;
+  const int nb = (int)(total_cells / (small ? YEE_TPB : YEE_CPB));
   cudaStream_t s = (cudaStream_t)stream;
-  if (prec == 0) k_yee_e_t<float><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, zero_j);
-  else k_yee_e_t<double><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, zero_j);
+#define PXRB_YEE(R_)                                                                            \
+  if (small) k_yee_e_t<R_, 1><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, zero_j);    \
+  else k_yee_e_t<R_, YEE_CPT><<<nb, YEE_TPB, 0, s>>>(jobs_dev, njobs, cell_off_dev, zero_j);
+  if (prec == 0) { PXRB_YEE(float) } else { PXRB_YEE(double) }
+#undef PXRB_YEE
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
 }
