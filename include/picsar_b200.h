@@ -87,6 +87,25 @@ int pxrb_geteb3d_energy_conserving(
     const double* byg, const double* bzg, int64_t ll4symtry, int64_t l_lower_order_in_v,
     int64_t lvect, int64_t field_gathe_algo, int64_t l_nodal, void* stream);
 
+/* Scratch bytes with which pxrb_geteb3d_energy_conserving_ws looks at the
+ * order of a call's particles and, if neighbours in memory are not neighbours
+ * in space, takes them by cell; 0 where that does not pay (orders 1 and 2, few
+ * particles).  The contents are not kept between calls.  Host function. */
+int64_t pxrb_order_scratch(int64_t order, int64_t np, int64_t nx, int64_t ny, int64_t nz,
+                           int64_t nxguard, int64_t nyguard, int64_t nzguard);
+
+/* The same with scratch (device, 4-byte aligned, at least pxrb_order_scratch
+ * bytes; NULL or less: particles as they come).  Same results. */
+int pxrb_geteb3d_energy_conserving_ws(
+    int64_t np, const double* xp, const double* yp, const double* zp, double* ex, double* ey,
+    double* ez, double* bx, double* by, double* bz, double xmin, double ymin, double zmin,
+    double dx, double dy, double dz, int64_t nx, int64_t ny, int64_t nz, int64_t nxguard,
+    int64_t nyguard, int64_t nzguard, int64_t nox, int64_t noy, int64_t noz,
+    const double* exg, const double* eyg, const double* ezg, const double* bxg,
+    const double* byg, const double* bzg, int64_t ll4symtry, int64_t l_lower_order_in_v,
+    int64_t lvect, int64_t field_gathe_algo, int64_t l_nodal, void* scratch,
+    int64_t scratch_bytes, void* stream);
+
 /* Replaces pxr_boris_push_u_3d (src/particle_pushers/boris_pusher/boris_3d.F90:51). */
 int pxrb_boris_push_u_3d(int64_t np, double* uxp, double* uyp, double* uzp, double* gaminv,
                          const double* ex, const double* ey, const double* ez,

@@ -33,6 +33,9 @@ _SIGS = {
     "pxrb_field_gathering_plus_particle_pusher": "i i" + " p" * 13 + " d" * 7 + " i" * 6
     + " p" * 6 + " d d i i d i d s",
     "pxrb_group_scratch": "=i i i i i i i i i",
+    "pxrb_order_scratch": "=i i i i i i i i i",
+    "pxrb_geteb3d_energy_conserving_ws": "i" + " p" * 9 + " d" * 6 + " i" * 9 + " p" * 6
+    + " i i i i i p i s",
     "pxrb_geteb3d_energy_conserving": "i" + " p" * 9 + " d" * 6 + " i" * 9 + " p" * 6
     + " i i i i i s",
     "pxrb_boris_push_u_3d": "i" + " p" * 10 + " d d d d s",

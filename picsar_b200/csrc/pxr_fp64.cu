@@ -160,12 +160,18 @@ struct GEBParams {
 };
 
 template <int ORDER, bool LOWER>
-__global__ void __launch_bounds__(GTPB, geteb_blocks(ORDER, LOWER)) k_geteb(GEBParams p) {
+__global__ void __launch_bounds__(GTPB, geteb_blocks(ORDER, LOWER)) k_geteb(GEBParams p, GatherOrder order) {
   constexpr int N = ORDER + 1, DEG = LOWER ? ORDER - 1 : ORDER, S = DEG + 1;
-  const i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (i >= p.np) return;
-  const double x = (p.xp[i] - p.xmin) * p.dxi, y = (p.yp[i] - p.ymin) * p.dyi,
-               z = (p.zp[i] - p.zmin) * p.dzi;
+  const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+  if (t >= p.np) return;
+  // asked for together with the flag that says whether it is the one to take
+  double px = p.xp[t], py = p.yp[t], pz = p.zp[t];
+  i64 i = t;
+  if (order.use && *order.use) {
+    i = order.perm[t];
+    px = p.xp[i]; py = p.yp[i]; pz = p.zp[i];
+  }
+  const double x = (px - p.xmin) * p.dxi, y = (py - p.ymin) * p.dyi, z = (pz - p.zmin) * p.dzi;
   NodeShape<ORDER, double> nx, ny, nz;
   StagDeg<DEG> sx, sy, sz;
   nx.set(x); ny.set(y); nz.set(z);
@@ -767,14 +773,15 @@ PXRB_FGP_N(2)
 PXRB_FGP_N(3)
 #undef PXRB_FGP_N
 
-int pxrb_geteb3d_energy_conserving(
+int pxrb_geteb3d_energy_conserving_ws(
     int64_t np, const double* xp, const double* yp, const double* zp, double* ex, double* ey,
     double* ez, double* bx, double* by, double* bz, double xmin, double ymin, double zmin,
     double dx, double dy, double dz, int64_t nx, int64_t ny, int64_t nz, int64_t nxguard,
     int64_t nyguard, int64_t nzguard, int64_t nox, int64_t noy, int64_t noz,
     const double* exg, const double* eyg, const double* ezg, const double* bxg,
     const double* byg, const double* bzg, int64_t ll4symtry, int64_t l_lower_order_in_v,
-    int64_t lvect, int64_t field_gathe_algo, int64_t l_nodal, void* stream) {
+    int64_t lvect, int64_t field_gathe_algo, int64_t l_nodal, void* scratch,
+    int64_t scratch_bytes, void* stream) {
   (void)lvect; (void)field_gathe_algo;
   if (np < 0) return PXRB_EINVAL;
   if (np == 0) return PXRB_OK;
@@ -791,13 +798,33 @@ int pxrb_geteb3d_energy_conserving(
   p.ss = l_nodal ? 0.0 : 0.5;
   cudaStream_t s = (cudaStream_t)stream;
   const int nb = nblocks(np, GTPB);
+  GatherOrder by_key = {nullptr, nullptr};
+  if (group_fits((int)nox, np, p.G, scratch, scratch_bytes)) {
+    const double lo[3] = {xmin, ymin, zmin}, di[3] = {p.dxi, p.dyi, p.dzi};
+    const int rc = gather_order((int)nox, np, xp, yp, zp, lo, di, p.G, scratch, s, by_key);
+    if (rc) return rc;
+  }
 #define PXRB_GEB(O_)                                                  \
-  if (l_lower_order_in_v) k_geteb<O_, true><<<nb, GTPB, 0, s>>>(p);    \
-  else k_geteb<O_, false><<<nb, GTPB, 0, s>>>(p);
+  if (l_lower_order_in_v) k_geteb<O_, true><<<nb, GTPB, 0, s>>>(p, by_key);    \
+  else k_geteb<O_, false><<<nb, GTPB, 0, s>>>(p, by_key);
   if (nox == 1) { PXRB_GEB(1) } else if (nox == 2) { PXRB_GEB(2) } else { PXRB_GEB(3) }
 #undef PXRB_GEB
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
+}
+
+int pxrb_geteb3d_energy_conserving(
+    int64_t np, const double* xp, const double* yp, const double* zp, double* ex, double* ey,
+    double* ez, double* bx, double* by, double* bz, double xmin, double ymin, double zmin,
+    double dx, double dy, double dz, int64_t nx, int64_t ny, int64_t nz, int64_t nxguard,
+    int64_t nyguard, int64_t nzguard, int64_t nox, int64_t noy, int64_t noz,
+    const double* exg, const double* eyg, const double* ezg, const double* bxg,
+    const double* byg, const double* bzg, int64_t ll4symtry, int64_t l_lower_order_in_v,
+    int64_t lvect, int64_t field_gathe_algo, int64_t l_nodal, void* stream) {
+  return pxrb_geteb3d_energy_conserving_ws(
+      np, xp, yp, zp, ex, ey, ez, bx, by, bz, xmin, ymin, zmin, dx, dy, dz, nx, ny, nz, nxguard,
+      nyguard, nzguard, nox, noy, noz, exg, eyg, ezg, bxg, byg, bzg, ll4symtry,
+      l_lower_order_in_v, lvect, field_gathe_algo, l_nodal, nullptr, 0, stream);
 }
 
 static int launch_push(int kind, int64_t np, double* ux, double* uy, double* uz, double* gi,

@@ -64,8 +64,28 @@ struct PosParams {
   double xmin, ymin, zmin, dxi, dyi, dzi;
 };
 
-template <int ORDER>
+// Whether a call's particles are in no useful order (the separate gather's
+// question): of 256 neighbours in memory, spread over the call by the golden
+// ratio (even steps can fall on row ends only), more than half lie further
+// apart than eight cells in x or one in y or z.  Every block asks the same
+// 256 pairs and clears its share of the counters if so.
+__global__ void __launch_bounds__(TPB) k_order_probe(PosParams p, Keys K, Scratch s) {
+  const double f = threadIdx.x * 0.6180339887498949;
+  const i64 i = (i64)((f - floor(f)) * (double)(p.np - 1)), j = min(i + 1, p.np - 1);
+  const double dx = floor((p.xp[j] - p.xmin) * p.dxi) - floor((p.xp[i] - p.xmin) * p.dxi);
+  const double dy = floor((p.yp[j] - p.ymin) * p.dyi) - floor((p.yp[i] - p.ymin) * p.dyi);
+  const double dz = floor((p.zp[j] - p.zmin) * p.dzi) - floor((p.zp[i] - p.zmin) * p.dzi);
+  const bool near = fabs(dx) <= 8.0 && fabs(dy) <= 1.0 && fabs(dz) <= 1.0;
+  const bool group = 2 * __syncthreads_count(!near) > TPB;
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.slow[1] = group;
+  if (group)
+    for (int k = blockIdx.x * TPB + threadIdx.x; k < K.nkeys; k += gridDim.x * TPB) s.cnt[k] = 0;
+}
+
+// COND: only if the probe found no order.
+template <int ORDER, bool COND>
 __global__ void __launch_bounds__(TPB) k_group_count(PosParams p, Keys K, Scratch s) {
+  if (COND && !s.slow[1]) return;
   for (i64 i = blockIdx.x * (i64)TPB + threadIdx.x; i < p.np; i += (i64)gridDim.x * TPB) {
     const int key = key_of<ORDER>(K, (p.xp[i] - p.xmin) * p.dxi, (p.yp[i] - p.ymin) * p.dyi,
                                   (p.zp[i] - p.zmin) * p.dzi);
@@ -101,7 +121,9 @@ __device__ __forceinline__ int block_exclusive(int v, int* sh, int& total) {
 }
 
 // counts -> exclusive prefixes within each chunk of keys, chunk totals
+template <bool COND>
 __global__ void __launch_bounds__(TPB) k_group_scan(Keys K, Scratch s) {
+  if (COND && !s.slow[1]) return;
   __shared__ int sh[32];
   constexpr int PER = CHUNK / TPB;
   const int base = blockIdx.x * CHUNK + threadIdx.x * PER;
@@ -122,7 +144,9 @@ __global__ void __launch_bounds__(TPB) k_group_scan(Keys K, Scratch s) {
 }
 
 // chunk totals -> exclusive prefixes (one block)
+template <bool COND>
 __global__ void __launch_bounds__(1024) k_group_scan_top(int nchunks, Scratch s) {
+  if (COND && !s.slow[1]) return;
   __shared__ int sh[32];
   int carry = 0;
   for (int b = 0; b < nchunks; b += 1024) {
@@ -135,7 +159,9 @@ __global__ void __launch_bounds__(1024) k_group_scan_top(int nchunks, Scratch s)
   if (threadIdx.x == 0) *s.slow = 0;
 }
 
+template <bool COND>
 __global__ void __launch_bounds__(TPB) k_group_perm(i64 np, Scratch s) {
+  if (COND && !s.slow[1]) return;
   for (i64 i = blockIdx.x * (i64)TPB + threadIdx.x; i < np; i += (i64)gridDim.x * TPB)
     s.perm[key_start(s, s.key[i]) + s.rank[i]] = (int)i;
 }
@@ -266,10 +292,24 @@ int group_particles(const PosParams& q, const Keys& K, const Scratch& s, cudaStr
   const int nch = (K.nkeys + CHUNK - 1) / CHUNK;
   if (cudaMemsetAsync(s.cnt, 0, sizeof(int) * (size_t)K.nkeys, st) != cudaSuccess)
     return PXRB_ELAUNCH;
-  k_group_count<ORDER><<<grid_of(q.np, TPB), TPB, 0, st>>>(q, K, s);
-  k_group_scan<<<nch, TPB, 0, st>>>(K, s);
-  k_group_scan_top<<<1, 1024, 0, st>>>(nch, s);
-  k_group_perm<<<grid_of(q.np, TPB), TPB, 0, st>>>(q.np, s);
+  k_group_count<ORDER, false><<<grid_of(q.np, TPB), TPB, 0, st>>>(q, K, s);
+  k_group_scan<false><<<nch, TPB, 0, st>>>(K, s);
+  k_group_scan_top<false><<<1, 1024, 0, st>>>(nch, s);
+  k_group_perm<false><<<grid_of(q.np, TPB), TPB, 0, st>>>(q.np, s);
+  return PXRB_OK;
+}
+
+// The same permutation for the separate gather, made only if
+// the particles are in no order (slow[1]).
+template <int ORDER>
+int order_particles(const PosParams& q, const Keys& K, const Scratch& s, cudaStream_t st) {
+  const int nch = (K.nkeys + CHUNK - 1) / CHUNK;
+  k_order_probe<<<148, TPB, 0, st>>>(q, K, s);
+  k_group_count<ORDER, true><<<grid_of(q.np, TPB), TPB, 0, st>>>(q, K, s);
+  k_group_scan<true><<<nch, TPB, 0, st>>>(K, s);
+  k_group_scan_top<true><<<1, 1024, 0, st>>>(nch, s);
+  k_group_perm<true><<<grid_of(q.np, TPB), TPB, 0, st>>>(q.np, s);
+  PXRB_CHECK_LAUNCH();
   return PXRB_OK;
 }
 
@@ -301,6 +341,20 @@ bool group_fits(int order, i64 np, const GridG& G, const void* scratch, i64 byte
          bytes >= 4 * scratch_ints(K, np) && (reinterpret_cast<uintptr_t>(scratch) & 3) == 0;
 }
 
+int gather_order(int order, i64 np, const double* xp, const double* yp, const double* zp,
+                 const double* lo, const double* di, const GridG& G, void* scratch,
+                 cudaStream_t st, GatherOrder& o) {
+  Keys K;
+  if (!make_keys(order, G.nx, G.ny, G.nz, G.gx, G.gy, G.gz, K)) return PXRB_EINVAL;
+  const Scratch s = carve(K, np, scratch);
+  PosParams q = {np, xp, yp, zp, lo[0], lo[1], lo[2], di[0], di[1], di[2]};
+  o.perm = s.perm;
+  o.use = s.slow + 1;
+  return order == 1 ? order_particles<1>(q, K, s, st)
+       : order == 2 ? order_particles<2>(q, K, s, st)
+                    : order_particles<3>(q, K, s, st);
+}
+
 int esirkepov_grouped(int order, const DepParams& p, void* scratch, cudaStream_t st) {
   Keys K;
   if (!make_keys(order, p.G.nx, p.G.ny, p.G.nz, p.G.gx, p.G.gy, p.G.gz, K)) return PXRB_EINVAL;
@@ -311,6 +365,26 @@ int esirkepov_grouped(int order, const DepParams& p, void* scratch, cudaStream_t
 }
 
 }  // namespace pxrd
+
+extern "C" int64_t pxrb_order_scratch(int64_t order, int64_t np, int64_t nx, int64_t ny,
+                                      int64_t nz, int64_t nxguard, int64_t nyguard,
+                                      int64_t nzguard) {
+  // Particles in no order, as they come -> by cell, microseconds, order 3:
+  // 1.97 M 1016 -> 400 (lower shapes) and 1463 -> 501 (full), 1.21 M 625 -> 208,
+  // 8.4 M 4342 -> 2755.  Order 2 gains up to 2 M (413 -> 337) and loses at 8.4 M
+  // (1746 -> 2692: the particles' nine columns no longer fit L2 and come in
+  // single sectors), order 1 always loses (133 -> 329).  Particles in order
+  // pay the probe and four kernels that return at once, 17 us: from 2^20
+  // particles on, where that is small.  (The fused gather + push moves 26
+  // columns per particle and by cell lost as much as it gained: 432 -> 903 at
+  // order 2, 1022 -> 955 at order 3, 1.97 M.)
+  Keys K;
+  if (order != 3 || np < (1 << 20) || np >= (1LL << 31) || nx < 0 || ny < 0 ||
+      nz < 0 || nxguard < 0 || nyguard < 0 || nzguard < 0 ||
+      !make_keys((int)order, nx, ny, nz, nxguard, nyguard, nzguard, K) || K.nkeys > np)
+    return 0;
+  return 4 * scratch_ints(K, np);
+}
 
 extern "C" int64_t pxrb_group_scratch(int64_t order, int64_t np, int64_t nx, int64_t ny,
                                       int64_t nz, int64_t nxguard, int64_t nyguard,

@@ -871,6 +871,19 @@ def field_gathering_plus_particle_pusher_3_3_3(*args, **kw):
     _fgp(3, *args, **kw)
 
 
+def _scratch(query, order, np_, nx, ny, nz, gx, gy, gz, device):
+    """(tensor, pointer, bytes) of the scratch a kernel takes for a call,
+    (None, None, 0) where it uses none."""
+    if np_ < 1 << 16:             # the queries' least size (spares small calls the query)
+        return None, None, 0
+    need = _lib.query(query, int(order), int(np_), int(nx), int(ny), int(nz), int(gx), int(gy),
+                      int(gz))
+    if need <= 0:
+        return None, None, 0
+    t = torch.empty(need, dtype=torch.uint8, device=device)
+    return t, t.data_ptr(), need
+
+
 def geteb3d_energy_conserving(np_, xp, yp, zp, ex, ey, ez, bx, by, bz, xmin, ymin, zmin, dx,
                               dy, dz, nx, ny, nz, nxguard, nyguard, nzguard, nox, noy, noz,
                               exg, eyg, ezg, bxg, byg, bzg, ll4symtry, l_lower_order_in_v,
@@ -878,11 +891,13 @@ def geteb3d_energy_conserving(np_, xp, yp, zp, ex, ey, ez, bx, by, bz, xmin, ymi
     """field_gathering_manager_3d.F90:295-323 (l_nodal = module l_nodalgrid)."""
     parts = [_ptr(a) for a in (xp, yp, zp, ex, ey, ez, bx, by, bz)]
     grids = [_ptr(a, grid=True) for a in (exg, eyg, ezg, bxg, byg, bzg)]
-    _lib.call("pxrb_geteb3d_energy_conserving", int(np_), *parts, float(xmin), float(ymin),
+    keep, scr, nscr = (_scratch("pxrb_order_scratch", nox, np_, nx, ny, nz, nxguard, nyguard,
+                                nzguard, exg.device) if nox == noy == noz else (None, None, 0))
+    _lib.call("pxrb_geteb3d_energy_conserving_ws", int(np_), *parts, float(xmin), float(ymin),
               float(zmin), float(dx), float(dy), float(dz), int(nx), int(ny), int(nz),
               int(nxguard), int(nyguard), int(nzguard), int(nox), int(noy), int(noz), *grids,
               int(bool(ll4symtry)), int(bool(l_lower_order_in_v)), int(lvect),
-              int(field_gathe_algo), int(bool(l_nodal)), _stream())
+              int(field_gathe_algo), int(bool(l_nodal)), scr, nscr, _stream())
 
 
 def pxr_boris_push_u_3d(np_, uxp, uyp, uzp, gaminv, ex, ey, ez, bx, by, bz, q, m, dt,
@@ -916,19 +931,6 @@ def pxr_pushxyz(np_, xp, yp, zp, uxp, uyp, uzp, gaminv, dt):
               float(dt), _stream())
 
 
-def _group_scratch(order, np_, nx, ny, nz, gx, gy, gz, device):
-    """(tensor, pointer, bytes) of the scratch the grouped deposition takes
-    for a call, (None, None, 0) where one particle per thread is used."""
-    if np_ < 1 << 16:             # pxrb_group_scratch is 0 (spares small calls the query)
-        return None, None, 0
-    need = _lib.query("pxrb_group_scratch", int(order), int(np_), int(nx), int(ny), int(nz),
-                      int(gx), int(gy), int(gz))
-    if need <= 0:
-        return None, None, 0
-    t = torch.empty(need, dtype=torch.uint8, device=device)
-    return t, t.data_ptr(), need
-
-
 def depose_jxjyjz(jx, jy, jz, np_, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin, ymin, zmin,
                   dt, dx, dy, dz, nx, ny, nz, nxguard, nyguard, nzguard, nox, noy, noz,
                   current_depo_algo=0, err_flag=None):
@@ -937,8 +939,8 @@ def depose_jxjyjz(jx, jy, jz, np_, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin
     own = err_flag is None
     if own:
         err_flag = torch.zeros(1, dtype=torch.int32, device=jx.device)
-    keep, scr, nscr = (_group_scratch(nox, np_, nx, ny, nz, nxguard, nyguard, nzguard, jx.device)
-                       if nox == noy == noz else (None, None, 0))
+    keep, scr, nscr = (_scratch("pxrb_group_scratch", nox, np_, nx, ny, nz, nxguard, nyguard,
+                                nzguard, jx.device) if nox == noy == noz else (None, None, 0))
     _lib.call("pxrb_depose_jxjyjz_ws", *[_ptr(a, grid=True) for a in (jx, jy, jz)], int(np_),
               *[_ptr(a) for a in (xp, yp, zp, uxp, uyp, uzp, gaminv, w)], float(q),
               float(xmin), float(ymin), float(zmin), float(dt), float(dx), float(dy), float(dz),

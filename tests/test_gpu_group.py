@@ -62,6 +62,31 @@ def test_deposit_matches_one_particle_per_thread(cuda, order, algo, np_, spread)
         assert float((a - b).abs().max()) <= 64 * per_node * 2.3e-16
 
 
+@pytest.mark.parametrize("order", [1, 2, 3])
+@pytest.mark.parametrize("np_,sort", [(20011, False), (20011, True), (997, False), (1, False)])
+def test_gather_by_cell_is_the_same(cuda, order, np_, sort):
+    """The separate gather with the ordering scratch (particles in no order,
+    and in cell order): the same bits, whichever way they are taken."""
+    n = (19, 13, 11)
+    x, u, w, fields = _inputs(n, np_, 30 * order, 0.4)
+    if sort:
+        by = torch.argsort((torch.floor(x[2]) * 64 + torch.floor(x[1])) * 64 + torch.floor(x[0]))
+        x = [a[by].contiguous() for a in x]
+    f = [a.data_ptr() for a in fields]
+    s = torch.cuda.current_stream().cuda_stream
+    out = []
+    for scr in (None, _scratch(order, np_, n)):
+        mem = (None, 0) if scr is None else (scr.data_ptr(), scr.numel())
+        eb = [torch.full_like(w, 0.25) for _ in range(6)]
+        for lower in (0, 1):
+            _lib.call("pxrb_geteb3d_energy_conserving_ws", np_, *[a.data_ptr() for a in x],
+                      *[a.data_ptr() for a in eb], 0.0, 0.0, 0.0, 1.0, 1.0, 1.0, *n, G, G, G,
+                      order, order, order, *f, 0, lower, 64, 0, 0, *mem, s)
+        out.append(eb)
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
 def test_scratch_rule(cuda):
     """No scratch where the grouped form is not used; enough where it is."""
     q = lambda np_, n: _lib.query("pxrb_group_scratch", 3, np_, n, n, n, 3, 3, 3)
