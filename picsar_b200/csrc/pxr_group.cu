@@ -47,7 +47,8 @@ template <int ORDER> __device__ __forceinline__ int base_cell(double x) {
   return ORDER == 2 ? fnint(x) : ffloor(x);
 }
 
-template <int ORDER> __device__ __forceinline__ int key_of(const Keys& K, double x, double y, double z) {
+template <int ORDER>
+__device__ __forceinline__ int key_of(const Keys& K, double x, double y, double z) {
   const int i = clampi(base_cell<ORDER>(x) + K.gx, K.nx) / Geom<ORDER>::C;
   const int j = clampi(base_cell<ORDER>(y) + K.gy, K.ny);
   const int k = clampi(base_cell<ORDER>(z) + K.gz, K.nz);
@@ -222,9 +223,13 @@ __global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K,
     double sy0[GE::N], sy1[GE::N], sz0[GE::N], sz1[GE::N];
     AX::shape(y - y0, sy0); AX::shape(yold - y0, sy1);
     AX::shape(z - z0, sz0); AX::shape(zold - z0, sz1);
-    const bool fast = valid && ok && oneoff;
+    // the products spread a group's operands over all of its nodes (0 times
+    // them): what is not finite keeps to the particle's own nodes in the list
+    const double cx = wq * p.invdtdx, cy = wq * p.invdtdy, cz = wq * p.invdtdz;
+    const bool fin = isfinite(x + xold + y + yold + z + zold) &&
+                     isfinite(fabs(cx) + fabs(cy) + fabs(cz));
+    const bool fast = valid && ok && oneoff && fin;
     if (valid && !fast) s.key[atomicAdd(s.slow, 1)] = ip;
-    const double f = fast ? wq : 0.0;
     if (!fast) {
       // no contribution: finite shapes times zero charge
 #pragma unroll
@@ -232,7 +237,7 @@ __global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K,
 #pragma unroll
       for (int t = 0; t < GE::N + 1; ++t) X.s0[t] = X.s1[t] = 0.0;
     }
-    J.stage(buf, X, sy0, sy1, sz0, sz1, f * p.invdtdx, f * p.invdtdy, f * p.invdtdz);
+    J.stage(buf, X, sy0, sy1, sz0, sz1, fast ? cx : 0.0, fast ? cy : 0.0, fast ? cz : 0.0);
     __syncwarp();
 #pragma unroll 1
     for (int t = 0; t < (n + 3) >> 2; ++t) J.sub(buf, t, X.i0 - (g.bx - GE::A));

@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
         int inc = v, ino = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, inc, o), x = __shfl_up_sync(0xffffffffu, ino, o);
+          const int u = __shfl_up_sync(0xffffffffu, inc, o);
+          const int x = __shfl_up_sync(0xffffffffu, ino, o);
           if (lane >= o) { inc += u; ino += x; }
         }
         if (k <= NKEY) { start[k] = run + inc - v; first[k] = oct + ino - w; }
@@ -214,12 +215,18 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
           sxs.set(ox); sys.set(oy); szs.set(oz);
           constexpr int N = GE::N, S = GE::S;
           const R* F0 = Fs + (vx + D + A) + (vy + D + A) * SY + (vz + D + A) * SZ;
-          eb[0] = gwin<S, N, N, SY, SZ>(F0 + sxs.r0 + nys.r0 * SY + nzs.r0 * SZ, sxs.s, nys.s, nzs.s);
-          eb[1] = gwin<N, S, N, SY, SZ>(F0 + V + nxs.r0 + sys.r0 * SY + nzs.r0 * SZ, nxs.s, sys.s, nzs.s);
-          eb[2] = gwin<N, N, S, SY, SZ>(F0 + 2 * V + nxs.r0 + nys.r0 * SY + szs.r0 * SZ, nxs.s, nys.s, szs.s);
-          eb[3] = gwin<N, S, S, SY, SZ>(F0 + 3 * V + nxs.r0 + sys.r0 * SY + szs.r0 * SZ, nxs.s, sys.s, szs.s);
-          eb[4] = gwin<S, N, S, SY, SZ>(F0 + 4 * V + sxs.r0 + nys.r0 * SY + szs.r0 * SZ, sxs.s, nys.s, szs.s);
-          eb[5] = gwin<S, S, N, SY, SZ>(F0 + 5 * V + sxs.r0 + sys.r0 * SY + nzs.r0 * SZ, sxs.s, sys.s, nzs.s);
+          eb[0] = gwin<S, N, N, SY, SZ>(F0 + sxs.r0 + nys.r0 * SY + nzs.r0 * SZ,
+                            sxs.s, nys.s, nzs.s);
+          eb[1] = gwin<N, S, N, SY, SZ>(F0 + V + nxs.r0 + sys.r0 * SY + nzs.r0 * SZ,
+                            nxs.s, sys.s, nzs.s);
+          eb[2] = gwin<N, N, S, SY, SZ>(F0 + 2 * V + nxs.r0 + nys.r0 * SY + szs.r0 * SZ,
+                            nxs.s, nys.s, szs.s);
+          eb[3] = gwin<N, S, S, SY, SZ>(F0 + 3 * V + nxs.r0 + sys.r0 * SY + szs.r0 * SZ,
+                            nxs.s, sys.s, szs.s);
+          eb[4] = gwin<S, N, S, SY, SZ>(F0 + 4 * V + sxs.r0 + nys.r0 * SY + szs.r0 * SZ,
+                            sxs.s, nys.s, szs.s);
+          eb[5] = gwin<S, S, N, SY, SZ>(F0 + 5 * V + sxs.r0 + sys.r0 * SY + nzs.r0 * SZ,
+                            sxs.s, sys.s, nzs.s);
         } else {
           gather_global<ORDER, R>(sj, ci, cj, ck, ox, oy, oz, eb);
         }
@@ -297,13 +304,17 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
       AX X;
       const bool okx = X.set(xn, x0, xo, x1);
       const bool todo = valid && !(pk & DONE);
-      const bool fast = todo && okx && sy + r0y == r1y && sz + r0z == r1z &&
+      // (what is not finite keeps to the particle's own nodes in the queue: the
+      // products spread a group's operands over all of its nodes)
+      const R cx = wgt * qdx, cy = wgt * qdy, cz = wgt * qdz;
+      const bool fin = isfinite(x0 + x1 + y0 + y1 + z0 + z1) &&
+                       isfinite(fabs(cx) + fabs(cy) + fabs(cz));
+      const bool fast = todo && okx && fin && sy + r0y == r1y && sz + r0z == r1z &&
                         (unsigned)(xn - x0c) < (unsigned)C;
       if (todo && !fast) q_list[pbeg + atomicAdd(&s_qn, 1)] = ip;
       R sy0[GE::N], sy1[GE::N], sz0[GE::N], sz1[GE::N];
       AX::shape(y0, sy0); AX::shape(y1, sy1);
       AX::shape(z0, sz0); AX::shape(z1, sz1);
-      const R wq = fast ? wgt : 0.0;
       if (!fast) {
         // no contribution: finite shapes times zero charge
 #pragma unroll
@@ -312,7 +323,7 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
         for (int t = 0; t < GE::N + 1; ++t) X.s0[t] = X.s1[t] = 0.0;
       }
       pxrg::Currents<ORDER> J;
-      J.stage(buf, X, sy0, sy1, sz0, sz1, wq * qdx, wq * qdy, wq * qdz);
+      J.stage(buf, X, sy0, sy1, sz0, sz1, fast ? cx : 0.0, fast ? cy : 0.0, fast ? cz : 0.0);
       __syncwarp();
       const int xoff = X.i0 + A - x0c;
       J.clear();
@@ -322,10 +333,10 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
         const int k = __shfl_sync(0xffffffffu, key, sub * 4);
         const int kn = __shfl_sync(0xffffffffu, key, min(sub * 4 + 4, 31));
         if (sub == 2 * nsub - 1 || kn != k) {
-          const int cx = (k % NG) * C;
-          double* base = Js + cx + ((k / NG) % NB) * SY + (k / (NG * NB)) * SZ;
+          const int col = (k % NG) * C;
+          double* base = Js + col + ((k / NG) % NB) * SY + (k / (NG * NB)) * SZ;
           J.flush([&](int c, int i, int j, int l, double v) {
-            if (v != 0.0 && cx + i < W) atomicAdd(base + c * V + i + j * SY + l * SZ, v);
+            if (v != 0.0 && col + i < W) atomicAdd(base + c * V + i + j * SY + l * SZ, v);
           });
           J.clear();
         }

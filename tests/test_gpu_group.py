@@ -63,6 +63,28 @@ def test_deposit_matches_one_particle_per_thread(cuda, order, algo, np_, spread)
 
 
 @pytest.mark.parametrize("order", [1, 2, 3])
+def test_deposit_of_weights_that_are_not_finite(cuda, order):
+    """An infinite or NaN weight reaches its particle's own nodes only, as with
+    one particle per thread."""
+    n, np_ = (19, 13, 11), 2000
+    x, u, w, _ = _inputs(n, np_, 40 + order, 0.4)
+    w[5], w[700], w[1500] = float("inf"), float("nan"), 1e308
+    gi = 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = []
+    for scr in (None, _scratch(order, np_, n)):
+        j = [P.grid_zeros(*n, G) for _ in range(3)]
+        _lib.call("pxrb_depose_jxjyjz_ws", *[a.data_ptr() for a in j], np_,
+                  *[a.data_ptr() for a in x + u], gi.data_ptr(), w.data_ptr(), -4.0, 0.0, 0.0,
+                  0.0, 0.5, 1.0, 1.0, 1.0, *n, G, G, G, order, order, order, 0, err.data_ptr(),
+                  None if scr is None else scr.data_ptr(), 0 if scr is None else scr.numel(),
+                  torch.cuda.current_stream().cuda_stream)
+        out.append(torch.stack(j))
+    a, b = (torch.isfinite(v) for v in out)
+    assert not bool(a.all()) and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3])
 @pytest.mark.parametrize("np_,sort", [(20011, False), (20011, True), (997, False), (1, False)])
 def test_gather_by_cell_is_the_same(cuda, order, np_, sort):
     """The separate gather with the ordering scratch (particles in no order,
