@@ -116,6 +116,17 @@ def _ng(a, n):
     return g2 // 2
 
 
+def _zero(*arrays):
+    """Clear arrays of one size: small ones in one launch (a fill each was 9 of
+    the 20 launches of a step on 16^3 cells, and that step is host-bound: 358 ->
+    335 us), large ones by a fill each (8.4 M particles: 70 us faster)."""
+    if arrays[0].numel() <= 1 << 18:
+        torch._foreach_zero_(list(arrays))
+    else:
+        for a in arrays:
+            a.zero_()
+
+
 # ---------------------------------------------------------------------------
 # Module state
 # ---------------------------------------------------------------------------
@@ -148,6 +159,10 @@ class Species:
     @property
     def np(self):
         return 0 if self.part_x is None else int(self.part_x.numel())
+
+    def zero_fields(self):
+        """Clear the particle field arrays (the gathers accumulate)."""
+        _zero(self.part_ex, self.part_ey, self.part_ez, self.part_bx, self.part_by, self.part_bz)
 
 
 _GRIDS = ("ex", "ey", "ez", "bx", "by", "bz", "jx", "jy", "jz", "rho", "dive")
@@ -274,8 +289,7 @@ class PicsarModule:
         for sp in self.species:
             if sp.np == 0:
                 continue
-            for c in ("ex", "ey", "ez", "bx", "by", "bz"):
-                getattr(sp, "part_" + c).zero_()
+            sp.zero_fields()
             fn(sp.np, sp.part_x, sp.part_y, sp.part_z, sp.part_ux, sp.part_uy, sp.part_uz,
                sp.part_gaminv, sp.part_ex, sp.part_ey, sp.part_ez, sp.part_bx, sp.part_by,
                sp.part_bz, self.xmin, self.ymin, self.zmin, self.dx, self.dy, self.dz, self.dt,
@@ -371,7 +385,7 @@ class PicsarModule:
         if self._tiled is not None:
             self._tiled.check_deposited()
             return
-        self.jx.zero_(); self.jy.zero_(); self.jz.zero_()
+        _zero(self.jx, self.jy, self.jz)
         for sp in self.species:
             if sp.np == 0 or not sp.ldodepos:
                 continue
@@ -880,7 +894,10 @@ def _scratch(query, order, np_, nx, ny, nz, gx, gy, gz, device):
                       int(gz))
     if need <= 0:
         return None, None, 0
-    t = torch.empty(need, dtype=torch.uint8, device=device)
+    try:
+        t = torch.empty(need, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None, None, 0      # the form without scratch serves any size
     return t, t.data_ptr(), need
 
 
@@ -1162,8 +1179,7 @@ class PicsarModule2D:
         for sp in self.species:
             if sp.np == 0:
                 continue
-            for c in ("ex", "ey", "ez", "bx", "by", "bz"):
-                getattr(sp, "part_" + c).zero_()
+            sp.zero_fields()
             geteb2dxz_energy_conserving(
                 sp.np, sp.part_x, sp.part_y, sp.part_z, sp.part_ex, sp.part_ey, sp.part_ez,
                 sp.part_bx, sp.part_by, sp.part_bz, self.xmin, 0.0, self.zmin, self.dx, 1.0,
@@ -1191,7 +1207,7 @@ class PicsarModule2D:
     def pxrdepose_currents_on_grid_jxjyjz(self):
         """J = 0, then the 2-D Esirkepov deposition of every species
         (current_deposition_manager_2d.F90:334)."""
-        self.jx.zero_(); self.jy.zero_(); self.jz.zero_()
+        _zero(self.jx, self.jy, self.jz)
         for sp in self.species:
             if sp.np == 0 or not sp.ldodepos:
                 continue
