@@ -38,7 +38,8 @@ extern "C" {
 #define PXRB_ETOOLARGE 6     /* job above the fixed limit of a no-allocation entry */
 
 /* ------------------------------------------------------------------------
- * Plain FP64 path (PICSAR arrays, one thread per particle, FP64 atomics)
+ * Plain FP64 path (PICSAR arrays; one thread per particle, FP64 atomics, and
+ * grouped forms that take the caller's scratch)
  * ---------------------------------------------------------------------- */
 
 /* Replaces field_gathering_plus_particle_pusher_{1_1_1,2_2_2,3_3_3}
@@ -453,8 +454,9 @@ typedef struct pxrb_tiled_job {
  * (particle_pusher_manager_3d.F90:1287-2193), particle_bcs (periodic,
  * particle_boundaries.F90:1109-1300) and depose_jxjyjz_esirkepov_{n}_{n}_{n}
  * (esirkepov_3d.F90:82, :1734, :3263).  Persistent CTAs pull (job, tile)
- * items; the tile's E/B window and J accumulator live in shared memory;
- * particles that left the window since the last sort take a global-memory
+ * items; the tile's E/B window and J accumulator live in shared memory (the
+ * FP64 engine at order 3 takes them one after the other and uses the sort's
+ * scratch perm, rank_b, cell_b and ox_b..oz_b); particles that left the window since the last sort take a global-memory
  * path.  jobs_dev: DEVICE descriptors (all of this `order` and `prec`);
  * work: DEVICE int32 pairs (job, tile), nwork of them (nwork_dev, if not
  * NULL, a DEVICE count <= nwork read at run time); ctr: DEVICE int32 reset by

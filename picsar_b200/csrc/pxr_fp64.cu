@@ -1,7 +1,8 @@
 // Plain FP64 path: the drop-in kernels behind PICSAR's Forthon-exposed
 // routines, on PICSAR's own guarded column-major FP64 arrays.  One thread per
-// particle; deposition uses global FP64 atomics.  This is also the "plain
-// FP64 GPU" baseline every mixed-precision / tiled speed-up is stated against.
+// particle; without scratch the deposition uses global FP64 atomics (with it,
+// pxr_group.cu).  This is also the "plain FP64 GPU" baseline every
+// mixed-precision / tiled speed-up is stated against.
 #include "pxr_fp64_dev.cuh"
 #include "picsar_b200.h"
 
