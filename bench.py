@@ -883,7 +883,8 @@ def run_plain_fp64(wl, args, ws, rank):
     return {"value": N * ws * args.fp64_steps / (ms * 1e-3), "unit": "particle-steps/s",
             "steps": args.fp64_steps, "ms_per_step": ms / args.fp64_steps,
             "what": "plain FP64 GPU path: PICSAR guarded FP64 arrays, one thread per "
-                    "particle, global FP64 atomics, separate bc kernels"}
+                    "particle for gather and push, deposit in groups (orders 2, 3), separate "
+                    "bc kernels"}
 
 
 def run_tiled_fp64(wl, args, ws, rank, cfg):
@@ -927,7 +928,7 @@ def run_tiled_fp64(wl, args, ws, rank, cfg):
                          "peak_kind": peak_kind, "algorithmic_bytes_per_launch": alg},
             "threads": c64.fp64_threads,
             "what": "tiled engine in FP64 (within 1e-12 of the oracle), same tiles and sort "
-                    "interval, no re-layout (the FP64 kernel makes one pass), one CTA per SM"}
+                    "interval, no re-layout (the FP64 kernel has no bank-class pass), one CTA per SM"}
 
 
 def _plain_fp64_jobs(specs, steps=2):
