@@ -39,7 +39,8 @@ template <int ORDER, int T, int D> struct TileGroups {
 
 // The current of a move from cell (ci, cj, ck), offsets o, by s cells to
 // offsets n, by global atomics (values only: arrays passed by address would
-// keep the caller's in local memory).
+// keep the caller's in local memory).  A move of more than one node (a step
+// beyond the CFL limit) sets the error flag.
 template <int ORDER>
 __device__ __noinline__ void deposit_outside(const Job& J, int ci, int cj, int ck, int sx, int sy,
                                              int sz, double ox, double oy, double oz, double nox,
@@ -55,7 +56,6 @@ __device__ __noinline__ void deposit_outside(const Job& J, int ci, int cj, int c
   esir_node<ORDER, R>(noz, r0, a0); esir_node<ORDER, R>(oz, r1, a1);
   ok = EZ.set(ck + sz + r0, a0, ck + r1, a1) && ok;
   if (!ok) atomicExch(&J.counters[1], 1);
-  atomicAdd(&J.counters[0], 1);
   dep_global<ORDER, R>(J, EX, EY, EZ, wgt * (J.q / (J.dt * J.dy * J.dz)),
                        wgt * (J.q / (J.dt * J.dx * J.dz)), wgt * (J.q / (J.dt * J.dx * J.dy)));
 }
@@ -252,14 +252,22 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
         ke += u2 / (1.0 + sqrt(u2 + 1.0)) * wgt;
         const bool in_new = in_old && vx + sx >= -D && vx + sx <= tex - 1 + D && vy + sy >= -D &&
                             vy + sy <= tey - 1 + D && vz + sz >= -D && vz + sz <= tez - 1 + D;
-        if (in_new) {
+        // the box word holds shifts of -1, 0 and 1: a longer move is deposited
+        // here, which flags it
+        const bool packs = sx >= -1 && sx <= 1 && sy >= -1 && sy <= 1 && sz >= -1 && sz <= 1;
+        if (in_new && packs) {
           q_pk[ip] = (unsigned)(vx + D + A) | ((unsigned)(vy + D + A) << 8) |
                      ((unsigned)(vz + D + A) << 16) | ((unsigned)(sx + 1) << 24) |
                      ((unsigned)(sy + 1) << 26) | ((unsigned)(sz + 1) << 28);
           q_ox[ip] = ox; q_oy[ip] = oy; q_oz[ip] = oz;
         } else {
           q_pk[ip] = DONE;
-          deposit_outside<ORDER>(sj, ci, cj, ck, sx, sy, sz, ox, oy, oz, nox, noy, noz, wgt);
+          if (!in_new) atomicAdd(&sj.counters[0], 1);
+          // a window particle's cell counted from its tile: its nodes before
+          // and after the move are then at most one period outside the grid
+          deposit_outside<ORDER>(sj, in_new ? c0x + vx : ci, in_new ? c0y + vy : cj,
+                                 in_new ? c0z + vz : ck, sx, sy, sz, ox, oy, oz, nox, noy, noz,
+                                 wgt);
         }
       }
     }

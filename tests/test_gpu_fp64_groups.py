@@ -3,7 +3,7 @@ its groups can go wrong."""
 import numpy as np
 import pytest
 
-from picsar_b200.tiled import TiledConfig
+from picsar_b200.tiled import TiledConfig, TiledSim
 from tests._cases import random_fields, rel_l2
 from tests.test_gpu_tiled import _pair
 
@@ -31,3 +31,24 @@ def test_tiled_fp64_groups_at_the_edges(cuda, n, tile, drift, crowd):
     assert t.error_flag() == 0
     for name in ("jx", "jy", "jz", "ex", "by"):
         assert rel_l2(t.export_field(name, 3).cpu().numpy(), o.get_field(name)) <= 1e-12, name
+
+
+@pytest.mark.parametrize("order", [1, 2, 3])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("cells", [0, -2, 3])
+def test_a_move_beyond_the_cfl_limit_is_flagged(cuda, order, axis, cells):
+    """A particle that moves by more than one cell a step inside its tile's
+    window sets the error flag; a step without one does not."""
+    n, dt, m = (16, 16, 16), 4.0, 300
+    rng = np.random.default_rng(order)
+    st = {c: rng.uniform(0, 16, m) for c in "xyz"}
+    st |= {"u" + c: 0.02 * rng.standard_normal(m) for c in "xyz"}
+    for q, c in enumerate("xyz"):
+        st[c][7] = 11.5
+        beta = (cells + 0.1 * np.sign(cells)) / dt if q == axis else 0.0
+        st["u" + c][7] = beta / np.sqrt(1 - beta * beta)
+    t = TiledSim(n, order=order, precision="fp64", dt=dt)
+    t.load_particles(*[st[c] for c in ("x", "y", "z", "ux", "uy", "uz")], np.ones(m))
+    assert t.job.dt == dt and (int(np.floor(11.5 + cells + 0.1 * np.sign(cells))) - 11) == cells
+    t.step(1)
+    assert (t.error_flag() != 0) == (cells != 0)
