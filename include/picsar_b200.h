@@ -410,8 +410,11 @@ typedef struct pxrb_tiled_job {
                                                kernel deferred to its second pass
                                                (bank classes taken); int32[4] */
   int32_t* cell_cnt;                        /* sort scratch: ntiles * tile^3 */
-  int32_t* rank_b;                          /* sort scratch: np */
-  int32_t* perm;                            /* sort scratch: np */
+  int32_t* rank_b;                          /* sort and step scratch: np (a step also
+                                               uses cell_b and ox_b..oz_b) */
+  int32_t* perm;                            /* sort scratch: np; step scratch too with
+                                               acc 5 and with select_lanes (which also
+                                               uses ux_b..uz_b) */
   float* tile_stats;                        /* NULL, or 4 per tile: the bounds of the
                                                fixed-point current scale for the
                                                next step (max |u|^2, max |w|, max
@@ -444,7 +447,11 @@ typedef struct pxrb_tiled_job {
  * load and sum their contributions to a J node before one atomic (tiles of
  * fewer than 2^21 particles: a larger tile sets the error flag and is left
  * unprocessed); jobs run with it set
- * `cell_order` so that the sort keeps cell order inside each tile.  The
+ * `cell_order` so that the sort keeps cell order inside each tile,
+ * 5 FP64 with the particle-grouped kernel (FP64 engine, shape order 3): each
+ * step puts a tile's particles into groups, in the job's perm, and sums a
+ * group's current on the FP64 matrix instruction; the E/B window and the J
+ * accumulator take the same shared memory one after the other.  The
  * fixed-point scales are bounded per tile from the tile's particle weights,
  * momenta, cell occupancy and fields, so no overflow is possible. */
 /* Fused per-step particle kernel of the tiled engine: energy-conserving
@@ -454,9 +461,8 @@ typedef struct pxrb_tiled_job {
  * (particle_pusher_manager_3d.F90:1287-2193), particle_bcs (periodic,
  * particle_boundaries.F90:1109-1300) and depose_jxjyjz_esirkepov_{n}_{n}_{n}
  * (esirkepov_3d.F90:82, :1734, :3263).  Persistent CTAs pull (job, tile)
- * items; the tile's E/B window and J accumulator live in shared memory (the
- * FP64 engine at order 3 takes them one after the other and uses the sort's
- * scratch perm, rank_b, cell_b and ox_b..oz_b); particles that left the window since the last sort take a global-memory
+ * items; the tile's E/B window and J accumulator live in shared memory;
+ * particles that left the window since the last sort take a global-memory
  * path.  jobs_dev: DEVICE descriptors (all of this `order` and `prec`);
  * work: DEVICE int32 pairs (job, tile), nwork of them (nwork_dev, if not
  * NULL, a DEVICE count <= nwork read at run time); ctr: DEVICE int32 reset by

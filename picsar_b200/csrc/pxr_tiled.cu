@@ -813,8 +813,8 @@ int64_t smem_bytes(int order, int prec, int acc, int tx, int ty, int tz, int dri
   const int lh = order == 1 ? 1 : 3, W = tx + 2 * drift + lh;
   const i64 V = (i64)pxrt::win_sz(tx, W) * W;
   i64 r = prec ? 8 : 4;
-  i64 a = acc == 3 ? 8 : 4, nw = acc == 2 ? 2 : 1;
-  if (prec == 1 && order == 3) {      // grouped FP64 kernel
+  i64 a = acc == 3 || acc == 5 ? 8 : 4, nw = acc == 2 ? 2 : 1;
+  if (acc == 5 && prec == 1 && order == 3) {      // particle-grouped FP64 kernel
     if (tx == 8 && drift == 1) return pxrt::TileGroups<3, 8, 1>::SMEM;
     if (tx == 8 && drift == 0) return pxrt::TileGroups<3, 8, 0>::SMEM;
     if (tx == 4 && drift == 1) return pxrt::TileGroups<3, 4, 1>::SMEM;

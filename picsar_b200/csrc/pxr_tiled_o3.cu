@@ -21,7 +21,7 @@ int launch_shape(int tile, int drift, int mode, const Job* jobs, const int2* wor
                  const int* nwork_dev, int* ctr, int threads, int ctas, size_t smem,
                  cudaStream_t s) {
 #define PXRB_TG(T_, D_)                                                                      \
-  if (tile == T_ && drift == D_ && mode == 3)                                               \
+  if (tile == T_ && drift == D_ && mode == 5)                                               \
     return launch_group<ORDER, T_, D_>(jobs, work, nwork, nwork_dev, ctr, threads, ctas, smem, s);
 #define PXRB_TD(T_, D_, M_)                                                                  \
   if (tile == T_ && drift == D_ && mode == M_)                                              \
@@ -38,6 +38,10 @@ int launch_shape(int tile, int drift, int mode, const Job* jobs, const int2* wor
     PXRB_TG(8, 0)
     PXRB_TG(4, 1)
     PXRB_TG(4, 0)
+    PXRB_TD(8, 1, 3)
+    PXRB_TD(8, 0, 3)
+    PXRB_TD(4, 1, 3)
+    PXRB_TD(4, 0, 3)
   } else {
     PXRB_TD(8, 1, 2)
     PXRB_TD(8, 1, 1)
@@ -67,5 +71,6 @@ int launch_order3(int prec, int tile, int drift, int mode, const pxrb_tiled_job*
 }  // namespace pxrt
 
 extern "C" int32_t pxrb_tiled_max_threads(int32_t acc) {
-  return acc == 4 ? pxrt::CG_THREADS : acc == 3 ? pxrt::MAX_THREADS_FP64 : pxrt::MAX_THREADS;
+  return acc == 4 ? pxrt::CG_THREADS
+       : acc == 3 || acc == 5 ? pxrt::MAX_THREADS_FP64 : pxrt::MAX_THREADS;
 }

@@ -83,15 +83,16 @@ _I32MAX = 2 ** 31 - 1
 SUPPORTED_SHAPES = {(8, 1), (8, 0), (8, 2), (4, 1), (4, 0)}
 # ... and those of the FP64 engine
 SUPPORTED_SHAPES_FP64 = {(8, 1), (8, 0), (4, 1), (4, 0)}
-# accumulator modes compiled for the FP32 engine per shape (FP64 engine: mode 3)
+# accumulator modes compiled for the FP32 engine per shape (FP64 engine: mode
+# 3, at shape order 3 the particle-grouped kernel, mode 5)
 SUPPORTED_ACC = {(8, 1): (0, 1, 2, 4), (8, 2): (1, 2), (4, 1): (1, 2)}
 
 
 def launch_threads(cfg, acc):
     """CTA size of the particle kernel for a configuration and accumulator:
-    `threads` for the FP32 engine, `fp64_threads` for the FP64 one (mode 3),
-    each at most pxrb_tiled_max_threads(acc)."""
-    want = cfg.fp64_threads if acc == 3 else cfg.threads
+    `threads` for the FP32 engine, `fp64_threads` for the FP64 one (modes 3
+    and 5), each at most pxrb_tiled_max_threads(acc)."""
+    want = cfg.fp64_threads if acc in (3, 5) else cfg.threads
     return min(want, _lib.query("pxrb_tiled_max_threads", acc))
 
 
@@ -192,7 +193,7 @@ class TiledSim:
         self.np = 0
         self.it = 0
         self.launches = 0          # kernels of this library launched so far
-        self.acc = 3 if self.prec == 1 else cfg.acc
+        self.acc = cfg.acc if self.prec == 0 else (5 if self.order == 3 else 3)
         if self.prec == 0 and self.acc not in SUPPORTED_ACC.get((tile[0], cfg.drift), (2,)):
             raise ValueError(f"accumulator mode {self.acc} not compiled for this tile shape")
         if self.acc == 4 and self.order == 2:

@@ -61,3 +61,14 @@ def test_max_threads_host():
     assert _lib.query("pxrb_tiled_max_threads", 1) == 256
     assert _lib.query("pxrb_tiled_max_threads", 4) == 256
     assert _lib.query("pxrb_tiled_max_threads", 3) == 512
+
+
+def test_fp64_modes_and_their_shared_memory():
+    """Mode 3 keeps the E/B and J windows of an FP64 tile side by side at every
+    order; the particle-grouped kernel is a mode of its own."""
+    from picsar_b200 import _lib
+    from picsar_b200.tiled import smem_bytes
+    assert [smem_bytes(o, 1, 3, (8, 8, 8), 1) for o in (1, 2, 3)] == [98208, 160992, 160992]
+    assert smem_bytes(3, 1, 3, (4, 4, 4), 1) == 67392
+    assert smem_bytes(3, 1, 5, (8, 8, 8), 1) != 160992
+    assert _lib.query("pxrb_tiled_max_threads", 5) == 512

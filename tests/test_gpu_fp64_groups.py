@@ -3,8 +3,8 @@ its groups can go wrong."""
 import numpy as np
 import pytest
 
-from picsar_b200.tiled import TiledConfig, TiledSim
-from tests._cases import random_fields, rel_l2
+from picsar_b200.tiled import TiledConfig, TiledSim, smem_bytes
+from tests._cases import plasma, random_fields, rel_l2
 from tests.test_gpu_tiled import _pair
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +52,20 @@ def test_a_move_beyond_the_cfl_limit_is_flagged(cuda, order, axis, cells):
     assert t.job.dt == dt and (int(np.floor(11.5 + cells + 0.1 * np.sign(cells))) - 11) == cells
     t.step(1)
     assert (t.error_flag() != 0) == (cells != 0)
+
+
+def test_one_pass_mode_takes_a_job_without_perm(cuda):
+    """Accumulator mode 3 at order 3 runs with its own window size and leaves
+    the sort's permutation alone."""
+    n = (16, 24, 16)
+    st = plasma(n, 3, 0.1, 11)
+    o, t = _pair(n, 3, 0, "fp64", st, TiledConfig(sort_interval=0, relayout_interval=0),
+                 random_fields(n, 3, 6))
+    assert t.acc == 5
+    t._pull_job()
+    t.acc, t.smem, t.job.perm = 3, smem_bytes(3, 1, 3, t.tile, t.cfg.drift), None
+    t._push_job()
+    o.step(2)
+    t.step(2, keep_j=True)
+    for name in ("jx", "jy", "jz", "ex", "by"):
+        assert rel_l2(t.export_field(name, 3).cpu().numpy(), o.get_field(name)) <= 1e-12, name
