@@ -495,9 +495,15 @@ int32_t pxrb_tiled_max_threads(int32_t acc);
 int64_t pxrb_tiled_job_size(void);
 
 /* Dynamic shared memory the particle kernel needs for a tile shape, order,
- * window margin and precision (host function, no GPU work). */
+ * window margin and precision, with any CTA size (host function, no GPU work). */
 int64_t pxrb_tiled_smem_bytes(int32_t order, int32_t prec, int32_t acc, int32_t tx,
                               int32_t ty, int32_t tz, int32_t drift);
+
+/* ... and the bytes of it that a launch of `threads` threads needs: less than
+ * pxrb_tiled_smem_bytes with acc 5 and fewer than 512 threads (host function;
+ * 0 for a bad CTA size). */
+int64_t pxrb_tiled_launch_smem(int32_t order, int32_t prec, int32_t acc, int32_t tile,
+                               int32_t drift, int32_t threads);
 
 /* Yee steps on the engine layout, every job in one launch (yee.F90:1258-1347
  * and :637-740; periodic guard images written by the same kernel).

@@ -65,7 +65,7 @@ def _key(order, precision, ppc, sigma, pusher, u_drift=0.0, device_name=None, ac
     sb = round(math.log10(max(sigma, 1e-6)) * 2) / 2
     db = f"|d{round(u_drift, 2)}" if u_drift else ""
     ab = f"|a{acc}" if precision == "fp32" else ""
-    return f"{name}|o{order}|{precision}|ppc{ppc}|s{sb}{db}|p{pusher}{ab}|v7"
+    return f"{name}|o{order}|{precision}|ppc{ppc}|s{sb}{db}|p{pusher}{ab}|v8"
 
 
 def acc_for(edge, drift, acc, order=3):

@@ -29,12 +29,16 @@ template <int ORDER, int T, int D> struct TileGroups {
   static constexpr int NB = T + 2 * D + (ORDER == 2 ? 1 : 0);
   static constexpr int NG = (NB + G::C - 1) / G::C;          // groups along x
   static constexpr int NKEY = NG * NB * NB;                  // and one more: outside the window
-  // the E/B window of the gather, then in its place the J window and the
-  // warps' records
+  // the E/B window of the gather, then in its place the J window and a record
+  // per lane of the launch's warps (edge 4 with 256 threads: 100,880 bytes, two
+  // CTAs per SM; records for 16 warps in any launch left it one)
   static constexpr int OFF_WIN = (2 * (NKEY + 2) * 4 + 15) / 16 * 16;
   static constexpr int OFF_BUF = OFF_WIN + (3 * V * 8 + 15) / 16 * 16;
-  static constexpr int END_J = OFF_BUF + MAX_WARPS * G::WARP_BYTES, END_F = OFF_WIN + 6 * V * 8;
-  static constexpr int SMEM = END_J > END_F ? END_J : END_F;
+  static constexpr int END_F = OFF_WIN + 6 * V * 8;
+  static constexpr int smem(int threads) {
+    const int end_j = OFF_BUF + threads / 32 * G::WARP_BYTES;
+    return end_j > END_F ? end_j : END_F;
+  }
 };
 
 // The current of a move from cell (ci, cj, ck), offsets o, by s cells to
@@ -413,12 +417,12 @@ template <int ORDER, int T, int D>
 int launch_group(const Job* jobs, const int2* work, int nwork, const int* nwork_dev, int* ctr,
                  int threads, int ctas, size_t smem, cudaStream_t s) {
   auto kern = k_tile_group<ORDER, T, D>;
-  if (smem < (size_t)TileGroups<ORDER, T, D>::SMEM) return PXRB_EINVAL;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
+  const int need = TileGroups<ORDER, T, D>::smem(threads);
+  if (smem < (size_t)need) return PXRB_EINVAL;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, need) != cudaSuccess)
     return PXRB_EUNSUPPORTED;
   if (cudaMemsetAsync(ctr, 0, sizeof(int), s) != cudaSuccess) return PXRB_ELAUNCH;
-  kern<<<ctas, threads, smem, s>>>(jobs, work, nwork, nwork_dev, ctr);
+  kern<<<ctas, threads, need, s>>>(jobs, work, nwork, nwork_dev, ctr);
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;
 }

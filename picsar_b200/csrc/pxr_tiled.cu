@@ -808,17 +808,17 @@ int diag_blocks(const Job& J) {
 template <int ORDER>
 constexpr int reach_total() { return Reach<ORDER>::L + Reach<ORDER>::H; }
 
-int64_t smem_bytes(int order, int prec, int acc, int tx, int ty, int tz, int drift) {
+int64_t smem_bytes(int order, int prec, int acc, int tx, int ty, int tz, int drift, int threads) {
   (void)ty; (void)tz;                 // cubic tiles
   const int lh = order == 1 ? 1 : 3, W = tx + 2 * drift + lh;
   const i64 V = (i64)pxrt::win_sz(tx, W) * W;
   i64 r = prec ? 8 : 4;
   i64 a = acc == 3 || acc == 5 ? 8 : 4, nw = acc == 2 ? 2 : 1;
   if (acc == 5 && prec == 1 && order == 3) {      // particle-grouped FP64 kernel
-    if (tx == 8 && drift == 1) return pxrt::TileGroups<3, 8, 1>::SMEM;
-    if (tx == 8 && drift == 0) return pxrt::TileGroups<3, 8, 0>::SMEM;
-    if (tx == 4 && drift == 1) return pxrt::TileGroups<3, 4, 1>::SMEM;
-    if (tx == 4 && drift == 0) return pxrt::TileGroups<3, 4, 0>::SMEM;
+    if (tx == 8 && drift == 1) return pxrt::TileGroups<3, 8, 1>::smem(threads);
+    if (tx == 8 && drift == 0) return pxrt::TileGroups<3, 8, 0>::smem(threads);
+    if (tx == 4 && drift == 1) return pxrt::TileGroups<3, 4, 1>::smem(threads);
+    if (tx == 4 && drift == 0) return pxrt::TileGroups<3, 4, 0>::smem(threads);
   }
   const i64 hb = tx + 2 * drift;      // next-step occupancy histogram (fixed point)
   if (acc == 4)                       // cell-grouped kernel (cg_smem_bytes)
@@ -840,7 +840,13 @@ int64_t pxrb_tiled_job_size(void) { return (int64_t)sizeof(pxrb_tiled_job); }
 
 int64_t pxrb_tiled_smem_bytes(int32_t order, int32_t prec, int32_t acc, int32_t tx, int32_t ty,
                               int32_t tz, int32_t drift) {
-  return smem_bytes(order, prec, acc, tx, ty, tz, drift);
+  return smem_bytes(order, prec, acc, tx, ty, tz, drift, pxrt::MAX_THREADS_FP64);
+}
+
+int64_t pxrb_tiled_launch_smem(int32_t order, int32_t prec, int32_t acc, int32_t tile,
+                               int32_t drift, int32_t threads) {
+  if (threads < 32 || threads > pxrt::MAX_THREADS_FP64) return 0;
+  return smem_bytes(order, prec, acc, tile, tile, tile, drift, threads);
 }
 
 int pxrb_tiled_particle_step(const pxrb_tiled_job* jobs_dev, int32_t order, int32_t prec,

@@ -60,6 +60,7 @@ _lib.register({
     "pxrb_tiled_field_export": "p I p i s",
     "pxrb_tiled_diagnostics": "p p p i p s",
     "pxrb_tiled_smem_bytes": "=i I I I I I I I",
+    "pxrb_tiled_launch_smem": "=i I I I I I I",
     "pxrb_tiled_job_size": "=i",
     "pxrb_tiled_max_threads": "I",
     "pxrb_tiled_diag_scratch": "=i p",

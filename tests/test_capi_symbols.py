@@ -72,3 +72,15 @@ def test_fp64_modes_and_their_shared_memory():
     assert smem_bytes(3, 1, 3, (4, 4, 4), 1) == 67392
     assert smem_bytes(3, 1, 5, (8, 8, 8), 1) != 160992
     assert _lib.query("pxrb_tiled_max_threads", 5) == 512
+
+
+def test_grouped_fp64_launches_share_an_sm():
+    """Two 256-thread CTAs of edge-4 tiles fit an SM's 227 KB in either FP64
+    mode (1 KB of it reserved and 1 KB of static memory per CTA)."""
+    from picsar_b200 import _lib
+    import picsar_b200.tiled  # noqa: F401
+    for acc in (3, 5):
+        need = [_lib.query("pxrb_tiled_launch_smem", 3, 1, acc, 4, 1, th) for th in (256, 512)]
+        assert 0 < need[0] <= need[1]
+        assert 2 * (need[0] + 2048) <= 227 * 1024, (acc, need)
+    assert _lib.query("pxrb_tiled_launch_smem", 3, 1, 5, 4, 1, 0) == 0

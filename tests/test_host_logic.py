@@ -67,6 +67,8 @@ def test_autotune_cache_keys():
     assert k() != k(sigma=0.05) and k() != k(ppc=16) and k() != k(order=2)
     assert k() != k(u_drift=0.2) and k(u_drift=0.2) == k(u_drift=0.2001)
     assert k().startswith("GPU|o3|fp32|ppc8|")
+    # choices timed on the FP64 kernels before the particle-grouped one are not served
+    assert not k(precision="fp64").endswith("|v7")
 
 
 def test_job_spec_rejects_jobs_without_steps():
