@@ -9,9 +9,12 @@
 // of x cells).  In that order the lanes of a warp read the same few window
 // elements, one wavefront a load, and a group's currents are added to the
 // tile's J window once per eight or more particles: 8.4 M particles at 8 per cell 3.73 ->
-// 2.92 ms, at 2 per cell (2.1 M) 1.31 -> 1.07 ms, at 1 per cell about even
-// (0.25 -> 0.27 ms at 64^3: the counting is then a sixth of the kernel).  What
-// is left is latency: one CTA fits an SM, so its phases do not overlap.
+// 2.95 ms, at 2 per cell (2.1 M) 1.31 -> 1.07 ms; at 1 per cell, not grouped,
+// 0.86 -> 0.68 ms.  What is left is latency: the warps' records leave room for
+// one CTA of 512 threads per SM, whose phases do not overlap, and for 28 KB of
+// L1, which particles outside their window miss (four fifths of them outside,
+// 8 per cell at 64^3: 12.0 ms against the one-pass kernel's 9.1; a plasma that
+// hot wants a shorter sort interval).
 // Orders 1 and 2 stay with k_tile_step (0.66 and 1.73 ms against 1.43 and 2.6
 // here): their 12 and 54 atomics cost less than the extra passes.
 #pragma once
@@ -25,10 +28,14 @@ template <int ORDER, int T, int D> struct TileGroups {
   static constexpr int L = Reach<ORDER>::L, H = Reach<ORDER>::H;
   static constexpr int W = T + 2 * D + L + H, SY = win_sy(T, W), SZ = win_sz(T, W), V = SZ * W;
   static_assert(L == G::A, "the window starts at the first cell's first node");
-  // base cells per axis (order 2: the nearest node may be one past the last cell)
-  static constexpr int NB = T + 2 * D + (ORDER == 2 ? 1 : 0);
+  static constexpr int NB = T + 2 * D;                       // base cells per axis
   static constexpr int NG = (NB + G::C - 1) / G::C;          // groups along x
   static constexpr int NKEY = NG * NB * NB;                  // and one more: outside the window
+  // Window particles per key below which a tile is not grouped.  Edge 8, margin
+  // 1, 512 threads, particle by particle / grouped: 0.68 / 0.91 ms at 1 per
+  // cell (2.6 per key), 1.21 / 1.08 ms at 2 (128x128x64 cells).  Edge 4 gains
+  // from the groups at any density (1 per cell, 256 threads 1.79 / 1.45 ms).
+  static constexpr int THIN = T == 8 ? 4 : 0;
   // the E/B window of the gather, then in its place the J window and a record
   // per lane of the launch's warps (edge 4 with 256 threads: 100,880 bytes, two
   // CTAs per SM; records for 16 warps in any launch left it one)
@@ -74,7 +81,7 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
   typedef EsirAxis<ORDER, R> AX;
   constexpr int SY = TG::SY, SZ = TG::SZ, V = TG::V, W = TG::W, NB = TG::NB, NG = TG::NG;
   constexpr int NKEY = TG::NKEY, C = GE::C, A = GE::A;
-  static_assert(NKEY + 1 <= MAX_THREADS_FP64, "one key per thread in the scan of the full CTA");
+  static_assert(ORDER == 3, "a particle's base cell is the cell that holds it");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int* start = reinterpret_cast<int*>(smem_raw);                   // counts, then starts
   int* first = start + NKEY + 2;                                   // first octet of a key
@@ -83,7 +90,7 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   double* buf = reinterpret_cast<double*>(smem_raw + TG::OFF_BUF + wid * GE::WARP_BYTES);
   __shared__ Job sj;
-  __shared__ int s_item, s_qn, s_key;
+  __shared__ int s_item, s_qn, s_key, s_grouped;
   __shared__ double s_red[MAX_WARPS];
 
   if (nwork_dev) nwork = min(nwork, *nwork_dev);
@@ -144,19 +151,17 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
       }
       asm volatile("cp.async.commit_group;\n" ::);
     }
-    // ---- groups: count (rank kept), prefix, placement ------------------------
+    // ---- groups: count (rank kept), prefix, placement; a thin tile and one
+    // that many particles have left is taken in storage order, its deposit by
+    // the queue ------------------------------------------------------------------
     // scratch free between sorts: rank_b (ranks, then the queue's list),
     // cell_b (keys, then the queue's boxes), perm (particles in group order)
     int *rank = sj.rank_b, *perm = sj.perm;
     uint32_t* keys = sj.cell_b;
-    for (int ip = pbeg + threadIdx.x; ip < pend; ip += blockDim.x) {
+    const bool dense = pend - pbeg >= TG::THIN * NKEY;
+    for (int ip = pbeg + threadIdx.x; dense && ip < pend; ip += blockDim.x) {
       int vx, vy, vz, key = NKEY;
-      if (local(cellp[ip], vx, vy, vz)) {
-        if (ORDER == 2) {
-          vx += oxp[ip] >= 0.5; vy += oyp[ip] >= 0.5; vz += ozp[ip] >= 0.5;
-        }
-        key = (vx + D) / C + NG * (vy + D + NB * (vz + D));
-      }
+      if (local(cellp[ip], vx, vy, vz)) key = (vx + D) / C + NG * (vy + D + NB * (vz + D));
       keys[ip] = (uint32_t)key;
       rank[ip] = atomicAdd(start + key, 1);
     }
@@ -178,10 +183,19 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
         run += __shfl_sync(0xffffffffu, inc, 31);
         oct += __shfl_sync(0xffffffffu, ino, 31);
       }
-      if (lane == 0) { start[NKEY + 1] = run; first[NKEY] = oct; }
+      __syncwarp();
+      if (lane == 0) {
+        // start[NKEY]: particles in the window.  Those outside read and add to
+        // global memory, in storage order with better locality than in the
+        // groups': with a quarter of them outside 16.8 / 15.6 ms (8 per cell,
+        // 64^3), with a third 16.7 / 11.3, with a sixth 16.3 / 19
+        s_grouped = dense && start[NKEY] >= TG::THIN * NKEY && 5 * start[NKEY] >= 4 * run;
+        start[NKEY + 1] = run;
+        first[NKEY] = s_grouped ? oct : 0;
+      }
     }
     __syncthreads();
-    for (int ip = pbeg + threadIdx.x; ip < pend; ip += blockDim.x)
+    for (int ip = pbeg + threadIdx.x; s_grouped && ip < pend; ip += blockDim.x)
       perm[pbeg + start[keys[ip]] + rank[ip]] = ip;
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
@@ -205,7 +219,7 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
     constexpr unsigned DONE = 1u << 31;
     {
       for (int s = threadIdx.x; s < pend - pbeg; s += blockDim.x) {
-        const int ip = perm[pbeg + s];
+        const int ip = s_grouped ? perm[pbeg + s] : pbeg + s;
         const uint32_t cell = cellp[ip];
         const R ox = oxp[ip], oy = oyp[ip], oz = ozp[ip];
         int ci, cj, ck, vx, vy, vz;
@@ -264,6 +278,7 @@ __global__ void __launch_bounds__(MAX_THREADS_FP64, 1)
                      ((unsigned)(vz + D + A) << 16) | ((unsigned)(sx + 1) << 24) |
                      ((unsigned)(sy + 1) << 26) | ((unsigned)(sz + 1) << 28);
           q_ox[ip] = ox; q_oy[ip] = oy; q_oz[ip] = oz;
+          if (!s_grouped) q_list[pbeg + atomicAdd(&s_qn, 1)] = ip;
         } else {
           q_pk[ip] = DONE;
           if (!in_new) atomicAdd(&sj.counters[0], 1);
