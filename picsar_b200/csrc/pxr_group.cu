@@ -23,6 +23,7 @@ using namespace pxrg;
 constexpr int TPB = 256, WARPS = TPB / 32;
 constexpr int CHUNK = 2048;                   // keys per scan block
 constexpr int SLOW_PAD = 32;                  // ints: the slow list's counter
+constexpr int SEG = 256;                      // particles of a group one warp takes
 
 // Group keys of a guarded grid: x groups fastest, then y and z base cells,
 // over every cell from -guard to n + guard.
@@ -37,7 +38,7 @@ struct Scratch {
   int *cnt;                                   // per key: count, then prefix in its chunk
   int *chunk;                                 // per chunk: prefix of the chunk totals
   int *key, *rank, *perm;                     // per particle
-  int *slow;                                  // counter, then (deposit) indices in `key`
+  int *slow;                                  // counter; the deposit's list is in `rank`
 };
 
 __device__ __forceinline__ int clampi(int v, int n) { return v < 0 ? 0 : (v >= n ? n - 1 : v); }
@@ -90,8 +91,13 @@ __global__ void __launch_bounds__(TPB) k_group_count(PosParams p, Keys K, Scratc
   for (i64 i = blockIdx.x * (i64)TPB + threadIdx.x; i < p.np; i += (i64)gridDim.x * TPB) {
     const int key = key_of<ORDER>(K, (p.xp[i] - p.xmin) * p.dxi, (p.yp[i] - p.ymin) * p.dyi,
                                   (p.zp[i] - p.zmin) * p.dzi);
+    // one atomic per warp and key: a crowded key's counter is one address
+    const unsigned act = __activemask(), peers = __match_any_sync(act, key);
+    const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
+    int base = 0;
+    if (lane == lead) base = atomicAdd(s.cnt + key, __popc(peers));
     s.key[i] = key;
-    s.rank[i] = atomicAdd(s.cnt + key, 1);
+    s.rank[i] = __shfl_sync(act, base, lead) + __popc(peers & ((1u << lane) - 1u));
   }
 }
 
@@ -167,37 +173,30 @@ __global__ void __launch_bounds__(TPB) k_group_perm(i64 np, Scratch s) {
     s.perm[key_start(s, s.key[i]) + s.rank[i]] = (int)i;
 }
 
-// A warp's group: its particles (range of the permutation), base cells of
-// column 0 and of y and z.
+// A group: its particles (range of the permutation), base cells of column 0
+// and of y and z.
 struct Group {
   int p0, p1, bx, by, bz;
 };
 template <int ORDER>
-__device__ __forceinline__ bool group_of(const Keys& K, const Scratch& s, i64 np, Group& g) {
-  const int key = blockIdx.x * WARPS + (threadIdx.x >> 5);
-  if (key >= K.nkeys) return false;
+__device__ __forceinline__ void group_of(const Keys& K, const Scratch& s, i64 np, int key, Group& g) {
   g.p0 = key_start(s, key);
   g.p1 = key + 1 < K.nkeys ? key_start(s, key + 1) : (int)np;
-  if (g.p0 >= g.p1) return false;
   const int r = key / K.nkx;
   g.bx = (key - r * K.nkx) * Geom<ORDER>::C - K.gx;
   g.by = r % K.ny - K.gy;
   g.bz = r / K.ny - K.gz;
-  return true;
 }
 
-// A particle whose y or z node changes, or whose x box leaves the group's
-// columns, goes to a list that one-particle-per-thread code works off after
-// (a few percent of a thermal plasma): inline it would cost its warp a whole
-// general deposit.
+// One warp's deposit of particles g.p0 .. g.p1 - 1 of a group.  A particle whose
+// y or z node changes, or whose x box leaves the group's columns, goes to a
+// list that one-particle-per-thread code works off after (a few percent of a
+// thermal plasma): inline it would cost its warp a whole general deposit.
 template <int ORDER>
-__global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K, Scratch s) {
+__device__ __forceinline__ void deposit_group(const DepParams& p, const Scratch& s, const Group& g,
+                                              double* buf) {
   typedef Geom<ORDER> GE;
   typedef EsirAxis<ORDER, double> AX;
-  extern __shared__ __align__(16) unsigned char smem[];
-  double* buf = reinterpret_cast<double*>(smem + (threadIdx.x >> 5) * GE::WARP_BYTES);
-  Group g;
-  if (!group_of<ORDER>(K, s, p.np, g)) return;               // whole warp
   const int lane = threadIdx.x & 31;
   Currents<ORDER> J;
   J.clear();
@@ -229,7 +228,7 @@ __global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K,
     const bool fin = isfinite(x + xold + y + yold + z + zold) &&
                      isfinite(fabs(cx) + fabs(cy) + fabs(cz));
     const bool fast = valid && ok && oneoff && fin;
-    if (valid && !fast) s.key[atomicAdd(s.slow, 1)] = ip;
+    if (valid && !fast) s.rank[atomicAdd(s.slow, 1)] = ip;
     if (!fast) {
       // no contribution: finite shapes times zero charge
 #pragma unroll
@@ -252,11 +251,45 @@ __global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K,
   });
 }
 
+// A group of at most SEG particles is one warp's.  A larger one (a beam, a thin
+// target: with a warp per group 2^20 particles in one cell took 77 ms, one
+// particle per thread 10.6) is cut at multiples of SEG of the permutation:
+// the first nseg warps each look at one such segment, which at most two large
+// groups can reach, and leave small groups to the warps after them.
+template <int ORDER>
+__global__ void __launch_bounds__(TPB, 2) k_esirkepov_group(DepParams p, Keys K, Scratch s, int nseg) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* buf = reinterpret_cast<double*>(smem + (threadIdx.x >> 5) * Geom<ORDER>::WARP_BYTES);
+  const int w = blockIdx.x * WARPS + (threadIdx.x >> 5);
+  const bool seg = w < nseg;
+  int lo = 0, hi = (int)p.np, key = w - nseg, last = key;
+  if (seg) {
+    lo = w * SEG;
+    hi = lo + min(hi - lo, SEG);
+    key = s.key[s.perm[lo]];
+    last = s.key[s.perm[hi - 1]];
+  } else if (key >= K.nkeys) {
+    return;                                                  // whole warp, as below
+  }
+#pragma unroll 1
+  for (;;) {
+    Group g;
+    group_of<ORDER>(K, s, p.np, key, g);
+    if (seg == (g.p1 - g.p0 > SEG) && g.p0 < g.p1) {
+      g.p0 = max(g.p0, lo);
+      g.p1 = min(g.p1, hi);
+      deposit_group<ORDER>(p, s, g, buf);
+    }
+    if (key == last) return;
+    key = last;
+  }
+}
+
 template <int ORDER>
 __global__ void __launch_bounds__(TPB) k_esirkepov_list(DepParams p, Scratch s) {
   const int n = *s.slow;
   for (int t = blockIdx.x * TPB + threadIdx.x; t < n; t += gridDim.x * TPB)
-    deposit_one<ORDER>(p, s.key[t]);
+    deposit_one<ORDER>(p, s.rank[t]);
 }
 
 int grid_of(i64 n, int tpb) {
@@ -329,7 +362,9 @@ int run_esirkepov(const DepParams& p, const Keys& K, const Scratch& s, cudaStrea
   const int smem = WARPS * Geom<ORDER>::WARP_BYTES;
   if (const int e = big_smem(k_esirkepov_group<ORDER>, smem)) return e;
   if (const int e = group_particles<ORDER>(q, K, s, st)) return e;
-  k_esirkepov_group<ORDER><<<(K.nkeys + WARPS - 1) / WARPS, TPB, smem, st>>>(p, K, s);
+  const int nseg = (int)((p.np + SEG - 1) / SEG);
+  const i64 warps = (i64)nseg + K.nkeys;
+  k_esirkepov_group<ORDER><<<(int)((warps + WARPS - 1) / WARPS), TPB, smem, st>>>(p, K, s, nseg);
   k_esirkepov_list<ORDER><<<148 * 4, TPB, 0, st>>>(p, s);
   PXRB_CHECK_LAUNCH();
   return PXRB_OK;

@@ -117,3 +117,54 @@ def test_scratch_rule(cuda):
     big = q(1 << 20, 64)
     assert big >= 4 * (3 * (1 << 20) + 71 * 71 * 15)
     assert np.iinfo(np.int32).max > big
+
+
+def _median_ms(f):
+    f()
+    took = []
+    for _ in range(5):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        f()
+        b.record()
+        torch.cuda.synchronize()
+        took.append(a.elapsed_time(b))
+    return sorted(took)[2]
+
+
+@pytest.mark.parametrize("order,cells", [(2, 1), (2, 10), (3, 1), (3, 10), (3, 1000)])
+def test_deposit_of_a_crowded_plasma(cuda, order, cells):
+    """2^20 particles in few cells through the public routine: the current of
+    one particle per thread, and in no more time (a warp per group took 7 to
+    10 times as long in one cell)."""
+    n, np_ = (64, 60, 56), 1 << 20
+    g = torch.Generator(device="cuda")
+    g.manual_seed(cells)
+    r = lambda: torch.rand(np_, generator=g, device="cuda", dtype=torch.float64)
+    corner = [(torch.rand(cells, generator=g, device="cuda") * (v - 1)).floor() for v in n]
+    pick = (r() * cells).long()
+    x = [c[pick].double() + r() for c in corner]
+    u = [0.2 + 0.05 * r() for _ in range(3)]
+    w = r() + 0.5
+    gi = 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert _lib.query("pxrb_group_scratch", order, np_, *n, G, G, G) > 0
+    js = [[P.grid_zeros(*n, G) for _ in range(3)] for _ in range(2)]
+    geom = (0.0, 0.0, 0.0, 0.5, 1.0, 1.0, 1.0, *n, G, G, G, order, order, order)
+
+    def grouped():
+        P.depose_jxjyjz(*js[0], np_, *x, *u, gi, w, -1.0, *geom, 0, err_flag=err)
+
+    def single():
+        _lib.call("pxrb_depose_jxjyjz", *[a.data_ptr() for a in js[1]], np_,
+                  *[a.data_ptr() for a in x + u], gi.data_ptr(), w.data_ptr(), -1.0, *geom, 0,
+                  err.data_ptr(), torch.cuda.current_stream().cuda_stream)
+
+    grouped()
+    single()
+    # currents of one sign: two sums of at most np_ terms, each within
+    # np_ * 2^-53 of its value
+    for a, b in zip(*js):
+        assert float((a - b).abs().max()) <= 2 * np_ * 2.0 ** -53 * float(b.abs().max())
+    assert int(err.item()) == 0
+    assert _median_ms(grouped) <= _median_ms(single)
