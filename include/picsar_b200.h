@@ -96,7 +96,8 @@ int64_t pxrb_order_scratch(int64_t order, int64_t np, int64_t nx, int64_t ny, in
                            int64_t nxguard, int64_t nyguard, int64_t nzguard);
 
 /* The same with scratch (device, 4-byte aligned, at least pxrb_order_scratch
- * bytes; NULL or less: particles as they come).  Same results. */
+ * bytes; NULL, less, or a call for which that is 0: particles as they come).
+ * Same results. */
 int pxrb_geteb3d_energy_conserving_ws(
     int64_t np, const double* xp, const double* yp, const double* zp, double* ex, double* ey,
     double* ez, double* bx, double* by, double* bz, double xmin, double ymin, double zmin,
@@ -155,8 +156,8 @@ int64_t pxrb_group_scratch(int64_t order, int64_t np, int64_t nx, int64_t ny, in
                            int64_t nxguard, int64_t nyguard, int64_t nzguard);
 
 /* The same with scratch (device, 4-byte aligned, at least pxrb_group_scratch
- * bytes; NULL or less: one particle per thread).  Sums within a group are made before the atomics, so J differs
- * by rounding. */
+ * bytes; NULL, less, or a call for which that is 0: one particle per thread).
+ * Sums within a group are made before the atomics, so J differs by rounding. */
 int pxrb_depose_jxjyjz_ws(double* jx, double* jy, double* jz, int64_t np, const double* xp,
                           const double* yp, const double* zp, const double* uxp,
                           const double* uyp, const double* uzp, const double* gaminv,

@@ -800,9 +800,9 @@ int pxrb_geteb3d_energy_conserving_ws(
   cudaStream_t s = (cudaStream_t)stream;
   const int nb = nblocks(np, GTPB);
   GatherOrder by_key = {nullptr, nullptr};
-  if (group_fits((int)nox, np, p.G, scratch, scratch_bytes)) {
+  if (order_fits((int)nox, np, p.G, scratch, scratch_bytes)) {
     const double lo[3] = {xmin, ymin, zmin}, di[3] = {p.dxi, p.dyi, p.dzi};
-    const int rc = gather_order((int)nox, np, xp, yp, zp, lo, di, p.G, scratch, s, by_key);
+    const int rc = gather_order(np, xp, yp, zp, lo, di, p.G, scratch, s, by_key);
     if (rc) return rc;
   }
 #define PXRB_GEB(O_)                                                  \

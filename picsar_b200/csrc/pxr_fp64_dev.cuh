@@ -114,18 +114,19 @@ __device__ __forceinline__ void deposit_one(const DepParams& p, i64 ip) {
   }
 }
 
-// Grouped form of the deposition and grouped order for the separate
-// gather // (pxr_group.cu).  group_fits: the scratch
-// serves the call.
+// Grouped form of the deposition and grouped order for the separate gather
+// (pxr_group.cu).  group_fits, order_fits: the call is one that
+// pxrb_group_scratch or pxrb_order_scratch asks scratch for, and this serves it.
 bool group_fits(int order, i64 np, const GridG& G, const void* scratch, i64 bytes);
-// The order in which the separate gather takes the call's particles: perm
-// where *use (device), else as they come.
+bool order_fits(int order, i64 np, const GridG& G, const void* scratch, i64 bytes);
+// The order in which the separate gather (order 3) takes the call's particles:
+// perm where *use (device), else as they come.
 struct GatherOrder {
   const int *perm, *use;
 };
-int gather_order(int order, i64 np, const double* xp, const double* yp, const double* zp,
-                 const double* lo, const double* di, const GridG& G, void* scratch,
-                 cudaStream_t st, GatherOrder& o);
+int gather_order(i64 np, const double* xp, const double* yp, const double* zp, const double* lo,
+                 const double* di, const GridG& G, void* scratch, cudaStream_t st,
+                 GatherOrder& o);
 int esirkepov_grouped(int order, const DepParams& p, void* scratch, cudaStream_t st);
 
 }  // namespace pxrd

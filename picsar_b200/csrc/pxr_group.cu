@@ -374,34 +374,33 @@ int run_esirkepov(const DepParams& p, const Keys& K, const Scratch& s, cudaStrea
 
 namespace pxrd {
 
+static bool fits(i64 need, const void* scratch, i64 bytes) {
+  return scratch && need > 0 && bytes >= need && (reinterpret_cast<uintptr_t>(scratch) & 3) == 0;
+}
 bool group_fits(int order, i64 np, const GridG& G, const void* scratch, i64 bytes) {
-  Keys K;
-  return scratch && np > 0 && np < (1LL << 31) &&
-         make_keys(order, G.nx, G.ny, G.nz, G.gx, G.gy, G.gz, K) &&
-         bytes >= 4 * scratch_ints(K, np) && (reinterpret_cast<uintptr_t>(scratch) & 3) == 0;
+  return fits(pxrb_group_scratch(order, np, G.nx, G.ny, G.nz, G.gx, G.gy, G.gz), scratch, bytes);
+}
+bool order_fits(int order, i64 np, const GridG& G, const void* scratch, i64 bytes) {
+  return fits(pxrb_order_scratch(order, np, G.nx, G.ny, G.nz, G.gx, G.gy, G.gz), scratch, bytes);
 }
 
-int gather_order(int order, i64 np, const double* xp, const double* yp, const double* zp,
-                 const double* lo, const double* di, const GridG& G, void* scratch,
-                 cudaStream_t st, GatherOrder& o) {
+int gather_order(i64 np, const double* xp, const double* yp, const double* zp, const double* lo,
+                 const double* di, const GridG& G, void* scratch, cudaStream_t st,
+                 GatherOrder& o) {
   Keys K;
-  if (!make_keys(order, G.nx, G.ny, G.nz, G.gx, G.gy, G.gz, K)) return PXRB_EINVAL;
+  if (!make_keys(3, G.nx, G.ny, G.nz, G.gx, G.gy, G.gz, K)) return PXRB_EINVAL;
   const Scratch s = carve(K, np, scratch);
   PosParams q = {np, xp, yp, zp, lo[0], lo[1], lo[2], di[0], di[1], di[2]};
   o.perm = s.perm;
   o.use = s.slow + 1;
-  return order == 1 ? order_particles<1>(q, K, s, st)
-       : order == 2 ? order_particles<2>(q, K, s, st)
-                    : order_particles<3>(q, K, s, st);
+  return order_particles<3>(q, K, s, st);
 }
 
 int esirkepov_grouped(int order, const DepParams& p, void* scratch, cudaStream_t st) {
   Keys K;
   if (!make_keys(order, p.G.nx, p.G.ny, p.G.nz, p.G.gx, p.G.gy, p.G.gz, K)) return PXRB_EINVAL;
   const Scratch s = carve(K, p.np, scratch);
-  return order == 1 ? run_esirkepov<1>(p, K, s, st)
-       : order == 2 ? run_esirkepov<2>(p, K, s, st)
-                    : run_esirkepov<3>(p, K, s, st);
+  return order == 2 ? run_esirkepov<2>(p, K, s, st) : run_esirkepov<3>(p, K, s, st);
 }
 
 }  // namespace pxrd
@@ -434,7 +433,16 @@ extern "C" int64_t pxrb_group_scratch(int64_t order, int64_t np, int64_t nx, int
   // order about even; 5.4 in order: 31 -> 66) and 65536 particles (110592 at
   // 16 per group: 84 -> 66); order 2 from 16 (17.7: 368 -> 267, 8.7: 138 ->
   // 127) and 131072 (110592: 39 -> 51); order 1, with 12 atomics per
-  // particle, never (8.4 M: 362 -> 561).
+  // particle, never (8.4 M: 362 -> 561).  These are cold plasmas.  In a hot one
+  // a third to half of the particles (u_th 0.5, 2) change their y or z node and
+  // are deposited on their own after all.  Order 3 in cell order 7.9 per group
+  // 958 -> 992 and 1071 -> 1235, 15.9 per group 2115 -> 1541 and 2345 -> 2014,
+  // in no order always faster; order 2 in cell order 18.5 per group 902 -> 906
+  // and 992 -> 1108, 37 per group 2130 -> 1588 and 2361 -> 1987, in no order
+  // 2087 -> 2233 and 2282 -> 2705.  (A probe of the momenta on the device that
+  // left such calls alone cost every call 10 us.)  Particles in few cells, in
+  // no order, 2^20 of them, order 3 / 2: one cell 10573 -> 286 / 7183 -> 239,
+  // a thousand 800 -> 192 / 341 -> 161.
   Keys K;
   const i64 least = order == 3 ? 1 << 16 : 1 << 17, per_key = order == 3 ? 6 : 16;
   if (order < 2 || order > 3 || np < least || np >= (1LL << 31) || nx < 0 || ny < 0 ||

@@ -29,6 +29,7 @@ namespace pxrg {
 constexpr int COLS = 8;                       // x nodes of a group
 
 template <int ORDER> struct Geom {
+  static_assert(ORDER == 2 || ORDER == 3, "two or three staggered nodes per axis");
   static constexpr int N = ORDER + 1;         // node-centred support
   static constexpr int S = ORDER;             // staggered support (one order lower)
   static constexpr int A = ORDER / 2;         // first support node: base cell - A
@@ -39,7 +40,7 @@ template <int ORDER> struct Geom {
   // the 16-byte stores of 8 lanes go to distinct banks (an even one made them
   // half of the shared-memory wavefronts), and 3 mod 8 leaves one conflict in
   // the 8 lanes' reads of 4 particles x 2 points.
-  static constexpr int DU = ORDER == 1 ? 11 : 19;
+  static constexpr int DU = 19;
   static constexpr int DZ = N, DX = 2 * N, DC = 2 * N + N + 1;    // unit offsets
   static constexpr int WARP_BYTES = 32 * DU * 16;
 };
@@ -121,13 +122,11 @@ template <int ORDER> struct Currents {
       if (2 * m + 1 < N || k < N) zk = o[G::DZ + k];
       dmma(jx[m], Py * zk.x + Qy * zk.y, bC);
     }
-    if (S >= 2) {
-      const double cy = c[h], cz = c[S + h];
-      dmma(ja, cy * Pz, bx.x);
-      dmma(ja, cy * Qz, bx.y);
-      dmma(jb, cz * Py, bx.x);
-      dmma(jb, cz * Qy, bx.y);
-    }
+    const double cy = c[h], cz = c[S + h];
+    dmma(ja, cy * Pz, bx.x);
+    dmma(ja, cy * Qz, bx.y);
+    dmma(jb, cz * Py, bx.x);
+    dmma(jb, cz * Qy, bx.y);
     if (S & 1) {
       const double cm = c[h * S + S - 1];
       dmma(jm, cm * (h ? Py : Pz), bx.x);
@@ -146,10 +145,8 @@ template <int ORDER> struct Currents {
 #pragma unroll
       for (int m = 0; m < G::XT; ++m)
         if (2 * m + 1 < N || h + 2 * m < N) put(0, i, t, h + 2 * m, jx[m][e]);
-      if (S >= 2) {
-        put(1, i, h, t, ja[e]);
-        put(2, i, t, h, jb[e]);
-      }
+      put(1, i, h, t, ja[e]);
+      put(2, i, t, h, jb[e]);
       if (S & 1) {
         if (h) put(2, i, t, S - 1, jm[e]);
         else put(1, i, S - 1, t, jm[e]);

@@ -1,7 +1,8 @@
-"""The grouped deposition (particles put into groups, FP64 matrix products) against one particle per thread, on the same inputs: odd
+"""The grouped deposition (particles put into groups, FP64 matrix products)
+and the gather by cell against one particle per thread on the same inputs: odd
 sizes, each order and pusher, particles in no order and in the guard cells,
 exact half-way positions, node changes along every axis, batches that are
-not full."""
+not full, crowded cells, and calls that the scratch rules leave alone."""
 import numpy as np
 import pytest
 import torch
@@ -31,74 +32,93 @@ def _inputs(n, np_, seed, spread):
     return x, u, w, fields
 
 
-def _scratch(order, np_, n):
-    # what pxrb_group_scratch would return without its size rule: an upper
-    # bound of keys, chunks and three ints per particle
-    keys = (n[0] + 2 * G + 8) * (n[1] + 2 * G + 1) * (n[2] + 2 * G + 1)
-    return torch.empty(4 * (2 * keys + 64 + 3 * np_) + 256, dtype=torch.uint8, device="cuda")
+GUARD = 0x5A
 
 
-@pytest.mark.parametrize("order", [1, 2, 3])
-@pytest.mark.parametrize("algo,np_,spread", [(0, 20011, 0.4), (1, 997, 1.5), (0, 1, 0.1)])
-def test_deposit_matches_one_particle_per_thread(cuda, order, algo, np_, spread):
+def _scratch(query, order, np_, n):
+    """The bytes a call asks for, and a pattern behind them."""
+    need = _lib.query(query, order, np_, *n, G, G, G)
+    assert need > 0
+    return torch.full((need + 4096,), GUARD, dtype=torch.uint8, device="cuda"), need
+
+
+def _thinned(x):
+    """Most particles in one octant, so that other groups hold few or none."""
+    half = x[0].numel() // 8 * 7
+    for a in x:
+        a[-half:] = a[-half:] / 2.0
+    return x
+
+
+@pytest.mark.parametrize("order,np_", [(2, 140011), (3, 70001)])
+@pytest.mark.parametrize("algo,spread", [(0, 0.4), (1, 1.5)])
+def test_deposit_matches_one_particle_per_thread(cuda, order, np_, algo, spread):
     n, dt = (19, 13, 11), 0.5
     x, u, w, _ = _inputs(n, np_, 20 * order + algo, spread)
+    x = _thinned(x)
     gi = 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    scr, need = _scratch("pxrb_group_scratch", order, np_, n)
     out = []
-    for scr in (None, _scratch(order, np_, n)):
+    for mem in ((None, 0), (scr.data_ptr(), need)):
         j = [P.grid_zeros(*n, G) for _ in range(3)]
         for a in j:
             a.fill_(0.125)                                  # the deposition accumulates
         _lib.call("pxrb_depose_jxjyjz_ws", *[a.data_ptr() for a in j], np_,
                   *[a.data_ptr() for a in x + u], gi.data_ptr(), w.data_ptr(), -1.0, 0.0, 0.0,
                   0.0, dt, 1.0, 1.0, 1.0, *n, G, G, G, order, order, order, algo, err.data_ptr(),
-                  None if scr is None else scr.data_ptr(), 0 if scr is None else scr.numel(),
-                  torch.cuda.current_stream().cuda_stream)
+                  *mem, torch.cuda.current_stream().cuda_stream)
         out.append(j)
     assert int(err.item()) == 0
-    per_node = max(1.0, np_ / (n[0] * n[1] * n[2]) * 64)
+    listed = int(scr[:4].view(torch.int32).item())
+    assert 0 < listed < np_                                 # grouped, some on their own
+    assert bool((scr[need:] == GUARD).all())
+    # a node sums at most the particles of the 5^3 cells around it (8 times the
+    # mean in the dense octant): two orders of the sum differ by at most twice
+    # that many terms times 2^-53 of the terms' sizes together, for which the
+    # largest current is the stricter stand-in (the terms partly cancel)
+    terms = 125 * 8 * np_ / (n[0] * n[1] * n[2])
     for a, b in zip(*out):
-        assert float((a - b).abs().max()) <= 64 * per_node * 2.3e-16
+        assert float((a - b).abs().max()) <= 2 * terms * 2.0 ** -53 * float(b.abs().max())
 
 
-@pytest.mark.parametrize("order", [1, 2, 3])
-def test_deposit_of_weights_that_are_not_finite(cuda, order):
+@pytest.mark.parametrize("order,np_", [(2, 140011), (3, 70001)])
+def test_deposit_of_weights_that_are_not_finite(cuda, order, np_):
     """An infinite or NaN weight reaches its particle's own nodes only, as with
     one particle per thread."""
-    n, np_ = (19, 13, 11), 2000
+    n = (19, 13, 11)
     x, u, w, _ = _inputs(n, np_, 40 + order, 0.4)
     w[5], w[700], w[1500] = float("inf"), float("nan"), 1e308
     gi = 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    scr, need = _scratch("pxrb_group_scratch", order, np_, n)
     out = []
-    for scr in (None, _scratch(order, np_, n)):
+    for mem in ((None, 0), (scr.data_ptr(), need)):
         j = [P.grid_zeros(*n, G) for _ in range(3)]
         _lib.call("pxrb_depose_jxjyjz_ws", *[a.data_ptr() for a in j], np_,
                   *[a.data_ptr() for a in x + u], gi.data_ptr(), w.data_ptr(), -4.0, 0.0, 0.0,
                   0.0, 0.5, 1.0, 1.0, 1.0, *n, G, G, G, order, order, order, 0, err.data_ptr(),
-                  None if scr is None else scr.data_ptr(), 0 if scr is None else scr.numel(),
-                  torch.cuda.current_stream().cuda_stream)
+                  *mem, torch.cuda.current_stream().cuda_stream)
         out.append(torch.stack(j))
     a, b = (torch.isfinite(v) for v in out)
     assert not bool(a.all()) and torch.equal(a, b)
 
 
-@pytest.mark.parametrize("order", [1, 2, 3])
-@pytest.mark.parametrize("np_,sort", [(20011, False), (20011, True), (997, False), (1, False)])
-def test_gather_by_cell_is_the_same(cuda, order, np_, sort):
-    """The separate gather with the ordering scratch (particles in no order,
-    and in cell order): the same bits, whichever way they are taken."""
-    n = (19, 13, 11)
+@pytest.mark.parametrize("sort", [False, True])
+def test_gather_by_cell_is_the_same(cuda, sort):
+    """The separate gather with the ordering scratch: the same bits for
+    particles in no order, which are taken by cell, and in cell order, which
+    are not."""
+    n, np_, order = (19, 13, 11), (1 << 20) + 5, 3
     x, u, w, fields = _inputs(n, np_, 30 * order, 0.4)
     if sort:
         by = torch.argsort((torch.floor(x[2]) * 64 + torch.floor(x[1])) * 64 + torch.floor(x[0]))
         x = [a[by].contiguous() for a in x]
     f = [a.data_ptr() for a in fields]
     s = torch.cuda.current_stream().cuda_stream
+    scr, need = _scratch("pxrb_order_scratch", order, np_, n)
     out = []
-    for scr in (None, _scratch(order, np_, n)):
-        mem = (None, 0) if scr is None else (scr.data_ptr(), scr.numel())
+    for mem in ((None, 0), (scr.data_ptr(), need)):
         eb = [torch.full_like(w, 0.25) for _ in range(6)]
         for lower in (0, 1):
             _lib.call("pxrb_geteb3d_energy_conserving_ws", np_, *[a.data_ptr() for a in x],
@@ -107,16 +127,38 @@ def test_gather_by_cell_is_the_same(cuda, order, np_, sort):
         out.append(eb)
     for a, b in zip(*out):
         assert torch.equal(a, b)
+    assert int(scr[4:8].view(torch.int32).item()) == int(not sort)     # the probe's answer
+    assert bool((scr[need:] == GUARD).all())
 
 
-def test_scratch_rule(cuda):
-    """No scratch where the grouped form is not used; enough where it is."""
-    q = lambda np_, n: _lib.query("pxrb_group_scratch", 3, np_, n, n, n, 3, 3, 3)
-    assert q(1000, 16) == 0
-    assert q(1 << 16, 512) == 0
-    big = q(1 << 20, 64)
-    assert big >= 4 * (3 * (1 << 20) + 71 * 71 * 15)
-    assert np.iinfo(np.int32).max > big
+def _calls(n, np_, order, x, u, w, fields, scr):
+    """The deposition and the gather of one call, on scratch `scr` (bytes)."""
+    gi = 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    j = [P.grid_zeros(*n, G) for _ in range(3)]
+    eb = [torch.zeros_like(w) for _ in range(6)]
+    s = torch.cuda.current_stream().cuda_stream
+    _lib.call("pxrb_depose_jxjyjz_ws", *[a.data_ptr() for a in j], np_,
+              *[a.data_ptr() for a in x + u], gi.data_ptr(), w.data_ptr(), -1.0, 0.0, 0.0, 0.0,
+              0.5, 1.0, 1.0, 1.0, *n, G, G, G, order, order, order, 0, err.data_ptr(),
+              scr.data_ptr(), scr.numel(), s)
+    _lib.call("pxrb_geteb3d_energy_conserving_ws", np_, *[a.data_ptr() for a in x],
+              *[a.data_ptr() for a in eb], 0.0, 0.0, 0.0, 1.0, 1.0, 1.0, *n, G, G, G, order,
+              order, order, *[a.data_ptr() for a in fields], 0, 1, 64, 0, 0, scr.data_ptr(),
+              scr.numel(), s)
+
+
+@pytest.mark.parametrize("order,np_", [(1, 200003), (2, 20011), (3, 20011), (3, 1)])
+def test_ample_scratch_does_not_change_the_rule(cuda, order, np_):
+    """A call for which the queries ask for no scratch leaves any it is given
+    alone, however large."""
+    n = (19, 13, 11)
+    x, u, w, fields = _inputs(n, np_, 50 + order, 0.4)
+    for q in ("pxrb_group_scratch", "pxrb_order_scratch"):
+        assert _lib.query(q, order, np_, *n, G, G, G) == 0
+    scr = torch.full((1 << 24,), GUARD, dtype=torch.uint8, device="cuda")
+    _calls(n, np_, order, x, u, w, fields, scr)
+    assert bool((scr == GUARD).all())
 
 
 def _median_ms(f):
