@@ -885,17 +885,17 @@ def field_gathering_plus_particle_pusher_3_3_3(*args, **kw):
     _fgp(3, *args, **kw)
 
 
-def _scratch(query, order, np_, nx, ny, nz, gx, gy, gz, device):
-    """(tensor, pointer, bytes) of the scratch a kernel takes for a call,
-    (None, None, 0) where it uses none."""
-    if np_ < 1 << 16:             # the queries' least size (spares small calls the query)
+def _scratch(query, order, np_, nx, ny, nz, gx, gy, gz, grid):
+    """(tensor, pointer, bytes) of the scratch a kernel takes for a call on
+    `grid`'s device, (None, None, 0) where it uses none."""
+    if np_ < 1 << 16 or grid is None:   # the queries' least size (spares small calls the query)
         return None, None, 0
     need = _lib.query(query, int(order), int(np_), int(nx), int(ny), int(nz), int(gx), int(gy),
                       int(gz))
     if need <= 0:
         return None, None, 0
     try:
-        t = torch.empty(need, dtype=torch.uint8, device=device)
+        t = torch.empty(need, dtype=torch.uint8, device=grid.device)
     except torch.cuda.OutOfMemoryError:
         return None, None, 0      # the form without scratch serves any size
     return t, t.data_ptr(), need
@@ -909,7 +909,7 @@ def geteb3d_energy_conserving(np_, xp, yp, zp, ex, ey, ez, bx, by, bz, xmin, ymi
     parts = [_ptr(a) for a in (xp, yp, zp, ex, ey, ez, bx, by, bz)]
     grids = [_ptr(a, grid=True) for a in (exg, eyg, ezg, bxg, byg, bzg)]
     keep, scr, nscr = (_scratch("pxrb_order_scratch", nox, np_, nx, ny, nz, nxguard, nyguard,
-                                nzguard, exg.device) if nox == noy == noz else (None, None, 0))
+                                nzguard, exg) if nox == noy == noz else (None, None, 0))
     _lib.call("pxrb_geteb3d_energy_conserving_ws", int(np_), *parts, float(xmin), float(ymin),
               float(zmin), float(dx), float(dy), float(dz), int(nx), int(ny), int(nz),
               int(nxguard), int(nyguard), int(nzguard), int(nox), int(noy), int(noz), *grids,
@@ -957,7 +957,7 @@ def depose_jxjyjz(jx, jy, jz, np_, xp, yp, zp, uxp, uyp, uzp, gaminv, w, q, xmin
     if own:
         err_flag = torch.zeros(1, dtype=torch.int32, device=jx.device)
     keep, scr, nscr = (_scratch("pxrb_group_scratch", nox, np_, nx, ny, nz, nxguard, nyguard,
-                                nzguard, jx.device) if nox == noy == noz else (None, None, 0))
+                                nzguard, jx) if nox == noy == noz else (None, None, 0))
     _lib.call("pxrb_depose_jxjyjz_ws", *[_ptr(a, grid=True) for a in (jx, jy, jz)], int(np_),
               *[_ptr(a) for a in (xp, yp, zp, uxp, uyp, uzp, gaminv, w)], float(q),
               float(xmin), float(ymin), float(zmin), float(dt), float(dx), float(dy), float(dz),

@@ -84,3 +84,17 @@ def test_grouped_fp64_launches_share_an_sm():
         assert 0 < need[0] <= need[1]
         assert 2 * (need[0] + 2048) <= 227 * 1024, (acc, need)
     assert _lib.query("pxrb_tiled_launch_smem", 3, 1, 5, 4, 1, 0) == 0
+
+
+def test_gather_of_no_particles_takes_no_arrays(monkeypatch):
+    """A call without particles needs none of its arrays (the library returns
+    before it looks at them); one with particles and no grid is refused by the
+    library."""
+    import pytest
+    from picsar_b200 import picsar as P
+    monkeypatch.setattr(P, "_stream", lambda: 0)
+    geom = (0.0, 0.0, 0.0, 1.0, 1.0, 1.0, 8, 8, 8, 3, 3, 3, 3, 3, 3)
+    args = [None] * 9, [None] * 6, (False, True, 64, 0)
+    P.geteb3d_energy_conserving(0, *args[0], *geom, *args[1], *args[2])
+    with pytest.raises(P.PicsarB200Error):
+        P.geteb3d_energy_conserving(1 << 20, *args[0], *geom, *args[1], *args[2])
