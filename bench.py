@@ -15,7 +15,9 @@ Arms:
   (default)          this framework; also reports the plain FP64 GPU path,
                      the end-to-end host-buffer run, the CPU oracle
                      baseline, a roofline of the fused particle kernel and
-                     the SM clocks sampled during the timed region.
+                     the SM clocks sampled during the timed region.  One
+                     JSON line on stdout; the whole record of every leg
+                     on stderr before it.
   --impl reference   the reference algorithm on the host CPU cores: the
                      C++ restatement of PICSAR's Fortran routines (the
                      Fortran itself cannot be compiled here), OpenMP over
@@ -506,6 +508,7 @@ def run_ours(args, emit=True):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
                          "kernel": (f"k_cell_step<{wl['order']}>" if cfg.acc == 4 else
+                                    "k_tile_group<3>" if prec == 1 and wl["order"] == 3 else
                                     f"k_tile_step<{'float' if prec == 0 else 'double'},"
                                     f"{wl['order']}>"),
                          "kernel_ms": kern_ms, "peak_kind": peak_kind,
@@ -527,11 +530,42 @@ def run_ours(args, emit=True):
         if ws == 1 and args.workload == "large" and not getattr(args, "skip_workloads", False):
             line["workloads"] = _workload_legs(args)
         if emit:
-            print(json.dumps(line), flush=True)
+            print(json.dumps(line), file=sys.stderr, flush=True)
+            print(json.dumps(headline(line)), flush=True)
     if ws > 1 and emit:
         import torch.distributed as dist
         dist.destroy_process_group()
     return line if rank == 0 else None
+
+
+# what the printed line keeps of its parts
+_HEADLINE = {
+    "config": ("workload", "precision", "particles_per_gpu", "cells", "parallelism", "l2"),
+    "roofline": ("bound", "achieved", "peak", "unit", "frac", "traffic", "kernel", "kernel_ms",
+                 "peak_kind", "algorithmic_bytes_per_launch"),
+    "cpu_baseline": ("value", "unit", "cores", "kind", "sample"),
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms"),
+    "clocks": ("sm_mhz", "sm_max_mhz", "reasons", "samples"),
+}
+
+
+def headline(line):
+    """The line printed on stdout: the headline, and of each other leg its
+    value alone, short enough to survive a reader that keeps the last 3000
+    characters.  (The whole record, accuracy and serving curves included, goes
+    to stderr before it.)"""
+    out = {}
+    for k, v in line.items():
+        if k in _HEADLINE and isinstance(v, dict):
+            out[k] = {q: v[q] for q in _HEADLINE[k] if q in v}
+        elif isinstance(v, dict) and k.startswith("fp64_"):
+            out[k] = {q: v[q] for q in ("value", "unit", "ms_per_step") if q in v}
+        elif isinstance(v, dict) and k == "workloads":
+            out[k] = {leg: {q: d[q] for q in ("value", "unit", "error") if q in d}
+                      for leg, d in v.items() if isinstance(d, dict)}
+        elif not isinstance(v, (dict, list)):
+            out[k] = v
+    return out
 
 
 def _compute_roofline(wl, prec, N, kern_ms):

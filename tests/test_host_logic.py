@@ -78,3 +78,27 @@ def test_job_spec_rejects_jobs_without_steps():
             JobSpec(n=(16, 16, 16), ppc=1, sigma=0.01, order=1, steps=bad)
     with pytest.raises(ValueError):
         JobSpec(n=(16, 0, 16), ppc=1, sigma=0.01, order=1)
+
+
+def test_bench_line_is_short():
+    """The benchmark's stdout line holds the headline, whatever the legs
+    report, within the 3000 characters a log's tail keeps."""
+    import json
+
+    import bench
+    leg = {"value": 1.0e10, "unit": "particle-steps/s", "curve": list(range(3000))}
+    desc = bench.WORKLOADS["uneven"]["desc"]
+    line = {"metric": "particle-steps/s", "value": 123456789.123456789, "n_gpus": 8,
+            "config": {"workload": desc, "precision": desc, "l2": desc, "tile_occupancy": leg},
+            "roofline": {"bound": "hbm", "kernel": desc, "extra": leg}, "compute_roofline": leg,
+            "cpu_baseline": {"value": 1.0, "sample": desc, "more": leg}, "accuracy": [leg],
+            "e2e": {"value": 2.0, "unit": "x", "h2d_bytes_per_step": 3, "what": desc * 9},
+            "clocks": {"sm_mhz": 1965, "reasons": []}, "fp64_plain": leg, "fp64_tiled": None,
+            "workloads": {k: leg for k in ("ensemble", "serve", "uneven")}}
+    short = bench.headline(line)
+    assert len(json.dumps(short)) < 2600
+    for k in ("metric", "value", "n_gpus", "fp64_tiled"):
+        assert short[k] == line[k]
+    assert short["e2e"] == {"value": 2.0, "unit": "x", "h2d_bytes_per_step": 3}
+    assert short["workloads"]["serve"] == {"value": 1.0e10, "unit": "particle-steps/s"}
+    assert "accuracy" not in short and "curve" not in json.dumps(short)
