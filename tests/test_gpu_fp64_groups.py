@@ -113,3 +113,19 @@ def test_particles_outside_their_window_are_not_grouped(cuda):
             took.append(ev[0].elapsed_time(ev[1]))
         ms[acc] = sorted(took)[2]
     assert ms[5] <= 1.45 * ms[3], ms
+
+
+def test_weights_that_are_not_finite_keep_to_their_nodes(cuda):
+    """The grouped kernel's sums leave an infinite or NaN weight on the nodes
+    the one-pass kernel puts it on."""
+    n, out = (16, 16, 16), []
+    st = thermal_plasma(n, 8, 0.05, seed=9, device="cuda")
+    st.w[5], st.w[20000], st.w[30001] = float("inf"), float("nan"), 1e308
+    for acc in (3, 5):
+        t = TiledSim(n, order=3, precision="fp64", q=-4.0)
+        t.acc, t.smem = acc, smem_bytes(3, 1, acc, t.tile, t.cfg.drift)
+        t.load_state(st)
+        t.particle_step()
+        out.append(torch.stack(t.J))
+    a, b = (torch.isfinite(v) for v in out)
+    assert 0 < int((~a).sum()) < 4000 and torch.equal(a, b)

@@ -210,3 +210,65 @@ def test_deposit_of_a_crowded_plasma(cuda, order, cells):
         assert float((a - b).abs().max()) <= 2 * np_ * 2.0 ** -53 * float(b.abs().max())
     assert int(err.item()) == 0
     assert _median_ms(grouped) <= _median_ms(single)
+
+
+def _shuffled(n, np_, seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    r = lambda: torch.rand(np_, generator=g, device="cuda", dtype=torch.float64)
+    x = [r() * v for v in n]
+    u = [0.1 + 0.05 * r() for _ in range(3)]
+    w = r() + 0.5
+    return x, u, w, 1.0 / torch.sqrt(1 + u[0] ** 2 + u[1] ** 2 + u[2] ** 2)
+
+
+@pytest.mark.parametrize("lower", [False, True])
+def test_public_gather_of_unsorted_particles(cuda, lower):
+    """geteb3d_energy_conserving above its rule's size: the bits of the entry
+    that takes no scratch (several scan chunks, grids that stride)."""
+    n, np_ = (64, 60, 56), (1 << 20) + 77
+    x, u, w, _ = _shuffled(n, np_, 3)
+    fields = []
+    for q in range(6):
+        f = P.grid_zeros(*n, G)
+        f.copy_(torch.randn(*f.shape, device="cuda", dtype=torch.float64))
+        fields.append(f)
+    assert _lib.query("pxrb_order_scratch", 3, np_, *n, G, G, G) > 0
+    a, b = ([torch.full_like(w, 0.5) for _ in range(6)] for _ in range(2))
+    geom = (0.0, 0.0, 0.0, 1.0, 1.0, 1.0, *n, G, G, G, 3, 3, 3)
+    P.geteb3d_energy_conserving(np_, *x, *a, *geom, *fields, False, lower, 64, 0)
+    _lib.call("pxrb_geteb3d_energy_conserving", np_, *[v.data_ptr() for v in x + b], *geom,
+              *[f.data_ptr() for f in fields], 0, int(lower), 64, 0, 0,
+              torch.cuda.current_stream().cuda_stream)
+    for p, q in zip(a, b):
+        assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("order", [2, 3])
+def test_public_deposition_with_and_without_memory(cuda, order, monkeypatch):
+    """depose_jxjyjz above its rule's size gives one current with scratch and,
+    when none can be had, without."""
+    n, np_ = (40, 36, 33), 1 << 20
+    x, u, w, gi = _shuffled(n, np_, 4)
+    assert _lib.query("pxrb_group_scratch", order, np_, *n, G, G, G) > 0
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def deposit():
+        j = [P.grid_zeros(*n, G) for _ in range(3)]
+        P.depose_jxjyjz(*j, np_, *x, *u, gi, w, -1.0, 0.0, 0.0, 0.0, 0.5, 1.0, 1.0, 1.0, *n, G, G,
+                        G, order, order, order, 0, err_flag=err)
+        return j
+
+    a, asked = deposit(), []
+
+    def no_memory(*size, **kw):
+        asked.append(size)
+        raise torch.cuda.OutOfMemoryError("none left")
+
+    monkeypatch.setattr(torch, "empty", no_memory)
+    b = deposit()
+    assert len(asked) == 1 and int(err.item()) == 0
+    # currents of one sign: sums of at most 125 cells' particles
+    terms = 125 * np_ / (n[0] * n[1] * n[2])
+    for p, q in zip(a, b):
+        assert float((p - q).abs().max()) <= 2 * terms * 2.0 ** -53 * float(q.abs().max())
