@@ -91,9 +91,14 @@ __global__ void __launch_bounds__(TPB) k_group_count(PosParams p, Keys K, Scratc
   for (i64 i = blockIdx.x * (i64)TPB + threadIdx.x; i < p.np; i += (i64)gridDim.x * TPB) {
     const int key = key_of<ORDER>(K, (p.xp[i] - p.xmin) * p.dxi, (p.yp[i] - p.ymin) * p.dyi,
                                   (p.zp[i] - p.zmin) * p.dzi);
-    // one atomic per warp and key: a crowded key's counter is one address
-    const unsigned act = __activemask(), peers = __match_any_sync(act, key);
-    const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
+    // one atomic per warp and key: a crowded key's counter is one address.  (In
+    // a warp whose first particle shares its key with no other, each on its
+    // own: particles in no order mostly differ, and matching them costs more.)
+    const unsigned act = __activemask();
+    const int lane = threadIdx.x & 31, k0 = __shfl_sync(act, key, __ffs(act) - 1);
+    const bool match = __popc(__ballot_sync(act, key == k0)) > 1;
+    const unsigned peers = match ? __match_any_sync(act, key) : 1u << lane;
+    const int lead = __ffs(peers) - 1;
     int base = 0;
     if (lane == lead) base = atomicAdd(s.cnt + key, __popc(peers));
     s.key[i] = key;
