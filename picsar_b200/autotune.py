@@ -6,7 +6,7 @@ For a (shape order, precision, particles per cell, thermal spread, beam
 drift) class of jobs, a proxy simulation large enough to occupy every SM (at least two tiles
 per resident CTA) is stepped under each candidate and timed with CUDA events
 on the launching stream.  Stage 1 times every compiled (tile edge, margin)
-pair at both thread counts (FP64: 256 and 512 threads, one CTA per SM)
+pair at both thread counts (FP64: 256 and 512 threads)
 over 20 steps with a sort every 5 steps; stage 2
 times the two best at each pair of sort interval and bank re-layout interval
 over 40 steps (the slow path for particles that drifted out of their tile
@@ -33,7 +33,7 @@ from ._lib import PicsarB200Error
 from .tiled import SUPPORTED_ACC, SUPPORTED_SHAPES, TiledConfig, TiledSim
 
 THREADS = (128, 256)
-THREADS_FP64 = (256, 512)     # the FP64 engine runs one CTA per SM
+THREADS_FP64 = (256, 512)     # the FP64 engine: one CTA per SM at edge 8
 SORT_INTERVALS = (5, 10, 20, 40)
 RELAYOUT_INTERVALS = (0, 2, 4)
 

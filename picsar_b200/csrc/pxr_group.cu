@@ -7,10 +7,10 @@
 // One particle per thread makes 144 global FP64 atomics per particle at order
 // 3 (0.19 T/s: 4.5 ms for 8.4 M particles at 8 per cell); a group of 40 makes
 // 240 together.  The grouping moves 24 B of position and 16 B of key, rank
-// and permutation per particle (0.17 ms of the 0.99 ms these 8.4 M take; 1.97 M
+// and permutation per particle (0.10 ms of the 0.97 ms these 8.4 M take; 1.97 M
 // particles in no order at 4 per cell: 1.27 -> 0.41 ms).  The shared-memory
-// pipe is the busiest unit then (records written and read back by other
-// lanes), with the FP64 pipe at half.
+// pipe is the busiest unit then (64 %: records written and read back by other
+// lanes), with the FP64 pipe at half (31 % DMMA, 21 % DFMA).
 #include "pxr_fp64_dev.cuh"
 #include "pxr_group.cuh"
 #include "picsar_b200.h"
@@ -342,8 +342,8 @@ int group_particles(const PosParams& q, const Keys& K, const Scratch& s, cudaStr
   return PXRB_OK;
 }
 
-// The same permutation for the separate gather, made only if
-// the particles are in no order (slow[1]).
+// The same permutation for the separate gather, made only if the particles
+// are in no order (slow[1]).
 template <int ORDER>
 int order_particles(const PosParams& q, const Keys& K, const Scratch& s, cudaStream_t st) {
   const int nch = (K.nkeys + CHUNK - 1) / CHUNK;

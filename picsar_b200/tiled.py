@@ -108,7 +108,7 @@ class TiledConfig:
     relayout_interval: int = 4  # bank-order re-layout of the tiles between sorts (0: none)
     acc: int = 2                # FP32 engine current accumulator (see picsar_b200.h)
     select_lanes: bool = True   # FP32 engine: distinct bank classes per warp, second pass
-    fp64_threads: int = 512     # FP64 engine's CTA size (one CTA per SM; `threads` is FP32's)
+    fp64_threads: int = 512     # FP64 engine's CTA size (one CTA per SM at edge 8; `threads`: FP32's)
 
 
 def h2d_bytes(buf):
