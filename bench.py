@@ -563,6 +563,11 @@ def headline(line):
         elif isinstance(v, dict) and k == "workloads":
             out[k] = {leg: {q: d[q] for q in ("value", "unit", "error") if q in d}
                       for leg, d in v.items() if isinstance(d, dict)}
+            for leg, d in v.items():                # a served stream: its highest rate
+                if isinstance(d, dict) and d.get("sweep"):
+                    out[k][leg] = {"value": d["sweep"][-1]["particle_steps_per_s"],
+                                   "unit": line["unit"],
+                                   "p99_latency_s": d["sweep"][-1]["p99_latency_s"]}
         elif not isinstance(v, (dict, list)):
             out[k] = v
     return out

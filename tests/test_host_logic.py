@@ -89,16 +89,19 @@ def test_bench_line_is_short():
     leg = {"value": 1.0e10, "unit": "particle-steps/s", "curve": list(range(3000))}
     desc = bench.WORKLOADS["uneven"]["desc"]
     line = {"metric": "particle-steps/s", "value": 123456789.123456789, "n_gpus": 8,
+            "unit": "particle-steps/s",
             "config": {"workload": desc, "precision": desc, "l2": desc, "tile_occupancy": leg},
             "roofline": {"bound": "hbm", "kernel": desc, "extra": leg}, "compute_roofline": leg,
             "cpu_baseline": {"value": 1.0, "sample": desc, "more": leg}, "accuracy": [leg],
             "e2e": {"value": 2.0, "unit": "x", "h2d_bytes_per_step": 3, "what": desc * 9},
             "clocks": {"sm_mhz": 1965, "reasons": []}, "fp64_plain": leg, "fp64_tiled": None,
-            "workloads": {k: leg for k in ("ensemble", "serve", "uneven")}}
+            "workloads": {"ensemble": leg, "uneven": leg, "serve": {"sweep": [
+                {"particle_steps_per_s": r, "p99_latency_s": 1.0} for r in (4.0, 5.0)]}}}
     short = bench.headline(line)
     assert len(json.dumps(short)) < 2600
     for k in ("metric", "value", "n_gpus", "fp64_tiled"):
         assert short[k] == line[k]
     assert short["e2e"] == {"value": 2.0, "unit": "x", "h2d_bytes_per_step": 3}
-    assert short["workloads"]["serve"] == {"value": 1.0e10, "unit": "particle-steps/s"}
+    assert short["workloads"]["ensemble"] == {"value": 1.0e10, "unit": "particle-steps/s"}
+    assert short["workloads"]["serve"]["value"] == 5.0
     assert "accuracy" not in short and "curve" not in json.dumps(short)
