@@ -432,9 +432,13 @@ template <int ORDER, int T, int D>
 int launch_group(const Job* jobs, const int2* work, int nwork, const int* nwork_dev, int* ctr,
                  int threads, int ctas, size_t smem, cudaStream_t s) {
   auto kern = k_tile_group<ORDER, T, D>;
-  const int need = TileGroups<ORDER, T, D>::smem(threads);
+  typedef TileGroups<ORDER, T, D> TG;
+  const int need = TG::smem(threads);
   if (smem < (size_t)need) return PXRB_EINVAL;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, need) != cudaSuccess)
+  // the limit of the largest launch, whatever this one needs: host threads that
+  // launch other CTA sizes set the same
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           TG::smem(MAX_THREADS_FP64)) != cudaSuccess)
     return PXRB_EUNSUPPORTED;
   if (cudaMemsetAsync(ctr, 0, sizeof(int), s) != cudaSuccess) return PXRB_ELAUNCH;
   kern<<<ctas, threads, need, s>>>(jobs, work, nwork, nwork_dev, ctr);

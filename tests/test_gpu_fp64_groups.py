@@ -129,3 +129,29 @@ def test_weights_that_are_not_finite_keep_to_their_nodes(cuda):
         out.append(torch.stack(t.J))
     a, b = (torch.isfinite(v) for v in out)
     assert 0 < int((~a).sum()) < 4000 and torch.equal(a, b)
+
+
+def test_cta_sizes_from_two_host_threads(cuda):
+    """Launches of different CTA sizes of one kernel, from two host threads on
+    their own streams, do not take each other's shared-memory limit."""
+    import threading
+    n, errors = (16, 16, 16), []
+
+    def run(threads):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                t = TiledSim(n, order=3, precision="fp64",
+                             config=TiledConfig(fp64_threads=threads, sort_interval=0))
+                t.load_state(thermal_plasma(n, 2, 0.05, seed=threads, device="cuda"))
+                for _ in range(300):
+                    t.particle_step()
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:                      # reported by the test's thread
+            errors.append(repr(e))
+
+    both = [threading.Thread(target=run, args=(k,)) for k in (128, 512)]
+    for b in both:
+        b.start()
+    for b in both:
+        b.join()
+    assert not errors
